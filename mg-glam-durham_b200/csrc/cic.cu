@@ -25,6 +25,7 @@
 #include "mgg_internal.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace mgg {
 
@@ -80,76 +81,133 @@ __global__ void k_cic_scatter(const float* __restrict__ x, const float* __restri
 }
 
 // One CTA per TY x TZ block of output rows (all N cells of each row), N = 2^lgN.
-// Shared memory: TY*TZ*N 64-bit accumulators (32 KB for 2 x 2 rows at N = 1024,
-// so several CTAs share an SM and hide each other's latency).
-constexpr int kDepTY = 2, kDepTZ = 2, kDepThreads = 256;
+// Shared memory: TY*TZ*N fixed-point accumulators of two 32-bit words each (64 KB for
+// 4 x 2 rows at N = 1024; several CTAs share an SM and hide each other's latency).
+// A 64-bit add to shared memory is a compare-and-swap loop, so a value v is added
+// as two 32-bit words: FIX_SPLIT, the low 20 bits and the rest, whose sums cannot
+// overflow while the CTA's list is short and the particles' weight small (most
+// lists; two adds that nothing waits for); FIX_CARRY, the low and high 32 bits, the
+// carry taken from the low word's old value; FIX_BIG the same for v >= 2^51 (a
+// handful of particles on the whole mesh).  Below 2^51 the integer is read off the
+// sum v + 2^52, which rounds as the conversion does.
+enum FixMode { FIX_SPLIT, FIX_CARRY, FIX_BIG };
+constexpr float kBigWpar = 131072.0f;   // particle weight from which v can reach 2^51
+template <FixMode MODE>
+__device__ __forceinline__ void fix_add(uint32_t* lo, uint32_t* hi, int cell, double v) {
+    const unsigned long long b = MODE == FIX_BIG ? __double2ull_rn(v)
+                                                 : (unsigned long long)__double_as_longlong(v + 4503599627370496.0);
+    const uint32_t l = (uint32_t)b, hw = (uint32_t)(b >> 32);
+    if (MODE == FIX_SPLIT) {
+        atomicAdd(lo + cell, l & 0xfffffu);
+        atomicAdd(hi + cell, __funnelshift_r(l, hw, 20));   // the exponent bits of v + 2^52 shift out
+        return;
+    }
+    const uint32_t old = atomicAdd(lo + cell, l);
+    const uint32_t h = (MODE == FIX_BIG ? hw : hw & 0xfffffu) + (old > ~l ? 1u : 0u);
+    if (h) atomicAdd(hi + cell, h);
+}
 
-template <int TY, int TZ>
-__global__ void __launch_bounds__(kDepThreads) k_cic_deposit(const float4* __restrict__ rec,
+// The source rows that reach the block are rows j0-1 .. j0+TY-1 of the planes k0-1 ..
+// k0+TZ-1; a plane's rows sit side by side in rec (two runs where j0-1 wraps), so
+// the block walks TZ+1 (or twice as many) runs as one list and no thread idles on a
+// short row.
+template <int TY, int TZ, int NT>
+__global__ void __launch_bounds__(NT) k_cic_deposit(const float4* __restrict__ rec,
                                                              const uint32_t* __restrict__ rowstart, int N, int lgN,
                                                              float wpar, float* __restrict__ fi) {
-    extern __shared__ unsigned long long acc[];
+    extern __shared__ uint32_t acc[];
+    constexpr int MAXRUN = 2 * (TZ + 1);
+    __shared__ uint32_t run_end[MAXRUN], run_off[MAXRUN];   // ends in the list; record - list position
     const int j0 = blockIdx.x * TY, k0 = blockIdx.y * TZ;
     const int nacc = (TY * TZ) << lgN;
-    for (int e = threadIdx.x; e < nacc; e += kDepThreads) acc[e] = 0ull;
-    __syncthreads();
-    const double W = (double)wpar;
-#pragma unroll 1
-    for (int sr = 0; sr < (TY + 1) * (TZ + 1); ++sr) {
-        int sj = j0 - 1 + sr % (TY + 1);
-        int sk = k0 - 1 + sr / (TY + 1);
-        sj = sj < 0 ? sj + N : sj;
-        sk = sk < 0 ? sk + N : sk;
-        const uint32_t row = (uint32_t)sj + ((uint32_t)sk << lgN);
-        const uint32_t beg = __ldg(rowstart + row), end = __ldg(rowstart + row + 1);
-        // target rows of this source row that fall inside the block
-        const int jj0 = sj - j0, jj1 = (sj + 1 == N ? 0 : sj + 1) - j0;
-        const int kk0 = sk - k0, kk1 = (sk + 1 == N ? 0 : sk + 1) - k0;
-        const bool vj0 = jj0 >= 0 && jj0 < TY, vj1 = jj1 >= 0 && jj1 < TY;
-        const bool vk0 = kk0 >= 0 && kk0 < TZ, vk1 = kk1 >= 0 && kk1 < TZ;
-        if (!((vj0 || vj1) && (vk0 || vk1))) continue;
-        for (uint32_t q = beg + threadIdx.x; q < end; q += kDepThreads) {
-            const float4 r = __ldg(rec + q);
-            const double X = r.x, Y = r.y, Z = r.z;
-            int I = (int)r.x;
-            I = I < 1 ? 1 : (I > N ? N : I);
-            const int Jc = (int)r.y, Kc = (int)r.z;
-            const double D1 = X - (double)(float)I, D2 = Y - (double)(float)Jc, D3 = Z - (double)(float)Kc;
-            const double T1 = 1.0 - D1, T2 = 1.0 - D2, T3 = 1.0 - D3;
-            const double T2W = T2 * W, D2W = D2 * W;
-            const int i0 = I - 1, i1 = (I == N) ? 0 : I;
-            if (vk0) {
-                if (vj0) {
-                    unsigned long long* a = acc + ((kk0 * TY + jj0) << lgN);
-                    atomicAdd(a + i0, __double2ull_rn(T3 * T1 * T2W * kFix));
-                    atomicAdd(a + i1, __double2ull_rn(T3 * D1 * T2W * kFix));
-                }
-                if (vj1) {
-                    unsigned long long* a = acc + ((kk0 * TY + jj1) << lgN);
-                    atomicAdd(a + i0, __double2ull_rn(T3 * T1 * D2W * kFix));
-                    atomicAdd(a + i1, __double2ull_rn(T3 * D1 * D2W * kFix));
-                }
-            }
-            if (vk1) {
-                if (vj0) {
-                    unsigned long long* a = acc + ((kk1 * TY + jj0) << lgN);
-                    atomicAdd(a + i0, __double2ull_rn(D3 * T1 * T2W * kFix));
-                    atomicAdd(a + i1, __double2ull_rn(D3 * D1 * T2W * kFix));
-                }
-                if (vj1) {
-                    unsigned long long* a = acc + ((kk1 * TY + jj1) << lgN);
-                    atomicAdd(a + i0, __double2ull_rn(D3 * T1 * D2W * kFix));
-                    atomicAdd(a + i1, __double2ull_rn(D3 * D1 * D2W * kFix));
-                }
-            }
+    uint32_t* lo = acc;
+    uint32_t* hi = acc + nacc;
+    for (int e = threadIdx.x; e < 2 * nacc; e += NT) acc[e] = 0u;
+    const bool wrap = j0 == 0;
+    const int nrun = wrap ? MAXRUN : TZ + 1;
+    if (threadIdx.x < 32) {
+        const int r = threadIdx.x;
+        uint32_t beg = 0, len = 0;
+        if (r < nrun) {
+            const int pl = wrap ? r >> 1 : r;
+            const int sk = (k0 - 1 + pl) & (N - 1);
+            const int first = wrap ? (r & 1 ? 0 : N - 1) : j0 - 1, last = wrap && !(r & 1) ? N - 1 : j0 + TY - 1;
+            beg = __ldg(rowstart + ((uint32_t)first + ((uint32_t)sk << lgN)));
+            len = __ldg(rowstart + ((uint32_t)last + ((uint32_t)sk << lgN) + 1)) - beg;
+        }
+        uint32_t end = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, end, o);
+            if (r >= o) end += y;
+        }
+        if (r < nrun) {
+            run_end[r] = end;
+            run_off[r] = beg - (end - len);
         }
     }
     __syncthreads();
+    const double W = (double)wpar * kFix;   // a power of two: the weights' bits are the unscaled ones
+    const uint32_t total = run_end[nrun - 1];
+    const bool split = total < 4096u && wpar * (float)total < 1048576.0f;
+    auto deposit = [&](auto mode) {
+      constexpr FixMode MODE = decltype(mode)::value;
+      for (uint32_t q = threadIdx.x; q < total; q += NT) {
+        int run = 0;
+        while (q >= run_end[run]) ++run;
+        const float4 r = __ldg(rec + (q + run_off[run]));
+        int I = (int)r.x;
+        I = I < 1 ? 1 : (I > N ? N : I);
+        int Jc = (int)r.y, Kc = (int)r.z;
+        const double D1 = (double)r.x - (double)(float)I, D2 = (double)r.y - (double)(float)Jc,
+                     D3 = (double)r.z - (double)(float)Kc;
+        const double T1 = 1.0 - D1, T2 = 1.0 - D2, T3 = 1.0 - D3;
+        const double T2W = T2 * W, D2W = D2 * W;
+        const int i0 = I - 1, i1 = (I == N) ? 0 : I;
+        // the bucket's row (a position clamped by the count sits in the clamped row)
+        Jc = Jc < 1 ? 1 : (Jc > N ? N : Jc);
+        Kc = Kc < 1 ? 1 : (Kc > N ? N : Kc);
+        // target rows inside the block
+        const int jj0 = Jc - 1 - j0, jj1 = (Jc == N ? 0 : Jc) - j0;
+        const int kk0 = Kc - 1 - k0, kk1 = (Kc == N ? 0 : Kc) - k0;
+        const bool vj0 = (unsigned)jj0 < (unsigned)TY, vj1 = (unsigned)jj1 < (unsigned)TY;
+        if ((unsigned)kk0 < (unsigned)TZ) {
+            const double a = T3 * T1, b = T3 * D1;
+            if (vj0) {
+                const int c = (kk0 * TY + jj0) << lgN;
+                fix_add<MODE>(lo, hi, c + i0, a * T2W);
+                fix_add<MODE>(lo, hi, c + i1, b * T2W);
+            }
+            if (vj1) {
+                const int c = (kk0 * TY + jj1) << lgN;
+                fix_add<MODE>(lo, hi, c + i0, a * D2W);
+                fix_add<MODE>(lo, hi, c + i1, b * D2W);
+            }
+        }
+        if ((unsigned)kk1 < (unsigned)TZ) {
+            const double a = D3 * T1, b = D3 * D1;
+            if (vj0) {
+                const int c = (kk1 * TY + jj0) << lgN;
+                fix_add<MODE>(lo, hi, c + i0, a * T2W);
+                fix_add<MODE>(lo, hi, c + i1, b * T2W);
+            }
+            if (vj1) {
+                const int c = (kk1 * TY + jj1) << lgN;
+                fix_add<MODE>(lo, hi, c + i0, a * D2W);
+                fix_add<MODE>(lo, hi, c + i1, b * D2W);
+            }
+        }
+      }
+    };
+    if (split) deposit(std::integral_constant<FixMode, FIX_SPLIT>{});
+    else if (wpar < kBigWpar) deposit(std::integral_constant<FixMode, FIX_CARRY>{});
+    else deposit(std::integral_constant<FixMode, FIX_BIG>{});
+    __syncthreads();
     const int64_t NN = (int64_t)N;
-    for (int e = threadIdx.x; e < nacc; e += kDepThreads) {
+    for (int e = threadIdx.x; e < nacc; e += NT) {
         const int i = e & (N - 1), rowl = e >> lgN;
         const int jj = rowl % TY, kk = rowl / TY;
-        const double v = (double)acc[e] * kUnfix - 1.0;
+        const double v = (double)(((unsigned long long)hi[e] << (split ? 20 : 32)) + lo[e]) * kUnfix - 1.0;
         fi[(int64_t)i + NN * ((int64_t)(j0 + jj) + NN * (int64_t)(k0 + kk))] = (float)v;
     }
 }
@@ -162,15 +220,20 @@ int ilog2i(int n) {
 
 // deposit launch for an N^3 grid (N a power of two, 16 <= N <= 1024)
 void launch_deposit(const float4* rec, const uint32_t* rowstart, int N, float wpar, float* fi, cudaStream_t s) {
-    const size_t smem = (size_t)kDepTY * kDepTZ * N * 8;   // <= 32 KB
-    k_cic_deposit<kDepTY, kDepTZ><<<dim3(N / kDepTY, N / kDepTZ), kDepThreads, smem, s>>>(rec, rowstart, N, ilog2i(N),
-                                                                                         wpar, fi);
+    // 4 x 2 rows a CTA visit a record 1.9 times on average, 2 x 2 rows 2.25 times, but small meshes need
+    // the CTAs: 2.95 -> 2.87 ms at 1024^3 (512^3 particles), 0.439 -> 0.420 at 512^3, equal at 256^3
+    if (N >= 512) {
+        k_cic_deposit<4, 2, 512><<<dim3(N / 4, N / 2), 512, (size_t)8 * N * 8, s>>>(rec, rowstart, N, ilog2i(N), wpar, fi);
+    } else {
+        k_cic_deposit<2, 2, 256><<<dim3(N / 2, N / 2), 256, (size_t)4 * N * 8, s>>>(rec, rowstart, N, ilog2i(N), wpar, fi);
+    }
 }
 
 }  // namespace
 
 void cic_alloc(Ctx& c) {
     const int64_t rows = (int64_t)c.N * c.N;
+    MGG_CUDA(cudaFuncSetAttribute(k_cic_deposit<4, 2, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     MGG_CUDA(cudaMalloc(&c.cic_rowcnt, sizeof(uint32_t) * (rows + 1)));
     MGG_CUDA(cudaMalloc(&c.cic_rowstart, sizeof(uint32_t) * (rows + 1)));
     MGG_CUDA(cudaMalloc(&c.cic_slot, sizeof(uint32_t) * c.np));
@@ -188,7 +251,10 @@ void cic_grid(Ctx& c, const float* x, const float* y, const float* z, int N, flo
         k_cic_count<<<blocks, threads, 0, c.stream>>>(x, y, z, c.np, N, c.cic_rowcnt, c.cic_slot, c.d_flags);
         MGG_CHECK_LAUNCH();
     }
-    scan_exclusive(c, c.cic_rowcnt, c.cic_rowstart, rows + 1);
+    {
+        ProfScope ps(c, K_SCAN, 8.0 * (double)(rows + 1));
+        scan_exclusive(c.cic_rowcnt, c.cic_rowstart, c.scan_tmp, rows + 1, c.stream);
+    }
     {
         ProfScope ps(c, K_CIC_SCATTER, 32.0 * c.np);
         k_cic_scatter<<<blocks, threads, 0, c.stream>>>(x, y, z, c.np, N, c.cic_rowstart, c.cic_slot, c.cic_rec);
@@ -281,56 +347,19 @@ constexpr int kNoAllocMaxNgrid = 256;
 constexpr int64_t kNoAllocMaxParticles = int64_t(1) << 21;
 constexpr size_t kNoAllocRows = (size_t)kNoAllocMaxNgrid * kNoAllocMaxNgrid + 1;
 constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
-constexpr size_t kNaOffRowcnt = 0;
+// the range flag sits before the row counts, so that one clear covers both; then the scan's block sums
+constexpr size_t kNaOffFlags = 0, kNaOffRowcnt = 256;
 constexpr size_t kNaOffRowstart = kNaOffRowcnt + align256(sizeof(uint32_t) * kNoAllocRows);
 constexpr size_t kNaOffSlot = kNaOffRowstart + align256(sizeof(uint32_t) * kNoAllocRows);
 constexpr size_t kNaOffRec = kNaOffSlot + align256(sizeof(uint32_t) * kNoAllocMaxParticles);
-constexpr size_t kNaOffFlags = kNaOffRec + align256(sizeof(float4) * kNoAllocMaxParticles);
-constexpr size_t kNoAllocBytes = kNaOffFlags + 256;
+constexpr size_t kNaOffSums = kNaOffRec + align256(sizeof(float4) * kNoAllocMaxParticles);
+constexpr size_t kNoAllocBytes = kNaOffSums + 256;   // 9 block sums at NGRID = 256
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 unsigned char* g_noalloc_ptr[kMaxDevices] = {};
-
-// Exclusive scan of n <= 65537 row counts by one CTA: chunks of 1024 with a
-// running carry (warp shuffles, then the warp totals).
-__global__ void __launch_bounds__(1024) k_scan_rows_1cta(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                         int64_t n) {
-    __shared__ uint32_t wsum[32];
-    __shared__ uint32_t carry;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    if (t == 0) carry = 0u;
-    for (int64_t base = 0; base < n; base += 1024) {
-        __syncthreads();
-        const int64_t g = base + t;
-        const uint32_t v = g < n ? in[g] : 0u;
-        uint32_t x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            uint32_t s = wsum[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-                if (lane >= o) s += y;
-            }
-            wsum[lane] = s;   // inclusive warp-total prefix
-        }
-        __syncthreads();
-        const uint32_t c0 = carry;
-        const uint32_t incl = x + (w > 0 ? wsum[w - 1] : 0u);
-        if (g < n) out[g] = c0 + incl - v;
-        __syncthreads();
-        if (t == 1023) carry = c0 + incl;
-    }
-}
 
 }  // namespace
 
@@ -370,12 +399,10 @@ void density_noalloc(const float* x, const float* y, const float* z, int64_t np,
     const int64_t rows = (int64_t)N * N;
     const int threads = 256;
     const int blocks = (int)std::min<int64_t>(div_up(np, threads), 148 * 16);
-    MGG_CUDA(cudaMemsetAsync(rowcnt, 0, sizeof(uint32_t) * (rows + 1), stream));
-    MGG_CUDA(cudaMemsetAsync(flags, 0, sizeof(int32_t), stream));
+    MGG_CUDA(cudaMemsetAsync(base, 0, kNaOffRowcnt + sizeof(uint32_t) * (rows + 1), stream));   // flag and counts
     k_cic_count<<<blocks, threads, 0, stream>>>(x, y, z, np, N, rowcnt, slot, flags);
     MGG_CHECK_LAUNCH();
-    k_scan_rows_1cta<<<1, 1024, 0, stream>>>(rowcnt, rowstart, rows + 1);
-    MGG_CHECK_LAUNCH();
+    scan_exclusive(rowcnt, rowstart, reinterpret_cast<uint32_t*>(base + kNaOffSums), rows + 1, stream);
     k_cic_scatter<<<blocks, threads, 0, stream>>>(x, y, z, np, N, rowstart, slot, rec);
     MGG_CHECK_LAUNCH();
     launch_deposit(rec, rowstart, N, (float)((double)N * N * N / (double)(float)np), fi, stream);

@@ -228,7 +228,7 @@ int mgg_create(const mgg_config* cfg, mgg_ctx** out) {
         alloc(&c.vx, c.np); alloc(&c.vy, c.np); alloc(&c.vz, c.np);
         fft_alloc(c);
         cic_alloc(c);
-        MGG_CUDA(cudaMalloc(&c.scan_tmp, sizeof(uint32_t) * 3 * 2048));
+        MGG_CUDA(cudaMalloc(&c.scan_tmp, sizeof(uint32_t) * 1024));
         MGG_CUDA(cudaMalloc(&c.d_flags, sizeof(int32_t)));
         MGG_CUDA(cudaMemset(c.d_flags, 0, sizeof(int32_t)));
         MGG_CUDA(cudaMalloc(&c.red_out, sizeof(double) * 4));

@@ -363,7 +363,8 @@ int background_table(mgg_config& c, double hubble, double* table, int capacity, 
 // reduce.cu helpers
 double reduce_sum_blocks(Ctx& c, int nblocks);   // sums red_partial[0..nblocks) on device, fixed order
 void reduce_sum_blocks_async(Ctx& c, int nblocks, double* out);   // the same sum into device memory, no wait
-void scan_exclusive(Ctx& c, const uint32_t* in, uint32_t* out, int64_t n);
+// exclusive sum of n counts (in, out 16-byte aligned; sums: one word per 8192 counts)
+void scan_exclusive(const uint32_t* in, uint32_t* out, uint32_t* sums, int64_t n, cudaStream_t s);
 void ensure_partials(Ctx& c, int n);
 
 // common constants

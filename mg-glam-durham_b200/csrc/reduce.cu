@@ -13,53 +13,84 @@ namespace mgg {
 
 namespace {
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 2 * kScanThreads;
+// The scan of the CIC row counts (up to 2^20 + 1 of them) is a latency chain, not a
+// bandwidth problem: 8192 counts per block (eight in a row per thread, then warp
+// shuffles), one launch up to 8192 counts and a second one that adds the totals of
+// the blocks before each block otherwise.
+constexpr int kScanThreads = 1024, kScanPer = 8, kScanItems = kScanThreads * kScanPer;
 
-// Block-local exclusive scan of 2048 uint32 (Blelloch in shared memory).
-__global__ void k_scan_block(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                             uint32_t* __restrict__ block_sums, int64_t n) {
-    __shared__ uint32_t s[kScanItems];
-    const int t = threadIdx.x;
-    const int64_t base = (int64_t)blockIdx.x * kScanItems;
-    const int64_t g0 = base + 2 * t, g1 = g0 + 1;
-    s[2 * t] = g0 < n ? in[g0] : 0u;
-    s[2 * t + 1] = g1 < n ? in[g1] : 0u;
-    int offset = 1;
-    for (int d = kScanItems >> 1; d > 0; d >>= 1) {
-        __syncthreads();
-        if (t < d) {
-            int ai = offset * (2 * t + 1) - 1, bi = offset * (2 * t + 2) - 1;
-            s[bi] += s[ai];
-        }
-        offset <<= 1;
+// exclusive sum of v over the block's threads; total: the block's sum (every thread)
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t& total) {
+    __shared__ uint32_t wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
+    if (lane == 31) wsum[w] = x;
     __syncthreads();
-    if (t == 0) {
-        if (block_sums) block_sums[blockIdx.x] = s[kScanItems - 1];
-        s[kScanItems - 1] = 0;
+    uint32_t t = wsum[lane];   // 32 warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) t += y;
     }
-    for (int d = 1; d < kScanItems; d <<= 1) {
-        offset >>= 1;
-        __syncthreads();
-        if (t < d) {
-            int ai = offset * (2 * t + 1) - 1, bi = offset * (2 * t + 2) - 1;
-            uint32_t tmp = s[ai];
-            s[ai] = s[bi];
-            s[bi] += tmp;
-        }
-    }
-    __syncthreads();
-    if (g0 < n) out[g0] = s[2 * t];
-    if (g1 < n) out[g1] = s[2 * t + 1];
+    total = __shfl_sync(0xffffffffu, t, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, t, w == 0 ? 0 : w - 1);
+    return x - v + (w == 0 ? 0u : before);
 }
 
-__global__ void k_scan_add(uint32_t* __restrict__ out, const uint32_t* __restrict__ block_off, int64_t n) {
-    const int64_t base = (int64_t)blockIdx.x * kScanItems;
-    const uint32_t add = block_off[blockIdx.x];
-    for (int e = threadIdx.x; e < kScanItems; e += blockDim.x) {
-        int64_t g = base + e;
-        if (g < n) out[g] += add;
+__global__ void __launch_bounds__(kScanThreads) k_scan_block(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                             uint32_t* __restrict__ block_sums, int64_t n) {
+    const int64_t g = (int64_t)blockIdx.x * kScanItems + kScanPer * threadIdx.x;
+    uint32_t v[kScanPer];
+    if (g + kScanPer <= n) {   // in and out are 16-byte aligned
+        const uint4 a = *reinterpret_cast<const uint4*>(in + g), b = *reinterpret_cast<const uint4*>(in + g + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanPer; ++i) v[i] = g + i < n ? in[g + i] : 0u;
+    }
+    uint32_t sum = 0;
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) {
+        const uint32_t t = v[i];
+        v[i] = sum;
+        sum += t;
+    }
+    uint32_t total;
+    const uint32_t base = block_scan(sum, total);
+    if (g + kScanPer <= n) {
+        *reinterpret_cast<uint4*>(out + g) = make_uint4(base + v[0], base + v[1], base + v[2], base + v[3]);
+        *reinterpret_cast<uint4*>(out + g + 4) = make_uint4(base + v[4], base + v[5], base + v[6], base + v[7]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanPer; ++i)
+            if (g + i < n) out[g + i] = base + v[i];
+    }
+    if (threadIdx.x == 0 && block_sums) block_sums[blockIdx.x] = total;
+}
+
+// adds the totals of blocks 0 .. blockIdx.x (of at most 1024) to block blockIdx.x + 1
+__global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t* __restrict__ out,
+                                                           const uint32_t* __restrict__ block_sums, int64_t n) {
+    uint32_t add;
+    block_scan(threadIdx.x <= blockIdx.x ? block_sums[threadIdx.x] : 0u, add);
+    const int64_t g = (int64_t)(blockIdx.x + 1) * kScanItems + kScanPer * threadIdx.x;
+    if (g + kScanPer <= n) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint4 a = *reinterpret_cast<uint4*>(out + g + 4 * h);
+            a.x += add; a.y += add; a.z += add; a.w += add;
+            *reinterpret_cast<uint4*>(out + g + 4 * h) = a;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kScanPer; ++i)
+            if (g + i < n) out[g + i] += add;
     }
 }
 
@@ -72,27 +103,13 @@ __global__ void k_sum_partials(const double* __restrict__ part, int n, double* _
 
 }  // namespace
 
-void scan_exclusive(Ctx& c, const uint32_t* in, uint32_t* out, int64_t n) {
-    ProfScope ps(c, K_SCAN, 8.0 * (double)n);
+void scan_exclusive(const uint32_t* in, uint32_t* out, uint32_t* sums, int64_t n, cudaStream_t s) {
     const int nb = div_up(n, kScanItems);
-    if (nb == 1) {
-        k_scan_block<<<1, kScanThreads, 0, c.stream>>>(in, out, nullptr, n);
-        MGG_CHECK_LAUNCH();
-        return;
-    }
-    if (nb > kScanItems * kScanItems) throw Error{MGG_ERR_ARG, "scan: too many elements"};
-    uint32_t* sums = c.scan_tmp;
-    uint32_t* sums_scan = c.scan_tmp + kScanItems * 2;
-    k_scan_block<<<nb, kScanThreads, 0, c.stream>>>(in, out, sums, n);
+    if (nb > kScanThreads) throw Error{MGG_ERR_ARG, "scan: too many elements"};
+    k_scan_block<<<nb, kScanThreads, 0, s>>>(in, out, sums, n);
     MGG_CHECK_LAUNCH();
-    const int nb2 = div_up(nb, kScanItems);
-    if (nb2 == 1) {
-        k_scan_block<<<1, kScanThreads, 0, c.stream>>>(sums, sums_scan, nullptr, nb);
-        MGG_CHECK_LAUNCH();
-    } else {
-        throw Error{MGG_ERR_ARG, "scan: more than 2048 blocks"};
-    }
-    k_scan_add<<<nb, 256, 0, c.stream>>>(out, sums_scan, n);
+    if (nb == 1) return;
+    k_scan_add<<<nb - 1, kScanThreads, 0, s>>>(out, sums, n);
     MGG_CHECK_LAUNCH();
 }
 
