@@ -206,22 +206,20 @@ LevelConsts make_consts(const Ctx& c, int l) {
 }
 
 // ------------------------------------------------------------- helpers -----
+// Periodic indices of a cell and its six neighbours (32 bits: n^3 <= 2^30, n a power of two)
 struct Nb {
-    int64_t c, xu, xl, yu, yl, zu, zl;
+    int c, xu, xl, yu, yl, zu, zl;
 };
 __device__ __forceinline__ Nb nb6(int i, int j, int k, int n) {
-    const int64_t nn = n;
-    const int iu = i + 1 == n ? 0 : i + 1, il = i == 0 ? n - 1 : i - 1;
-    const int ju = j + 1 == n ? 0 : j + 1, jl = j == 0 ? n - 1 : j - 1;
-    const int ku = k + 1 == n ? 0 : k + 1, kl = k == 0 ? n - 1 : k - 1;
+    const int m = n - 1, row = n * (j + n * k), pl = n * n;
     Nb r;
-    r.c = i + nn * (j + nn * k);
-    r.xu = iu + nn * (j + nn * k);
-    r.xl = il + nn * (j + nn * k);
-    r.yu = i + nn * (ju + nn * k);
-    r.yl = i + nn * (jl + nn * k);
-    r.zu = i + nn * (j + nn * ku);
-    r.zl = i + nn * (j + nn * kl);
+    r.c = row + i;
+    r.xu = row + ((i + 1) & m);
+    r.xl = row + ((i - 1) & m);
+    r.yu = i + n * (((j + 1) & m) + n * k);
+    r.yl = i + n * (((j - 1) & m) + n * k);
+    r.zu = i + n * j + pl * ((k + 1) & m);
+    r.zl = i + n * j + pl * ((k - 1) & m);
     return r;
 }
 
@@ -336,6 +334,102 @@ __device__ __forceinline__ double trig_root(double P, double Q, double D0, doubl
     return chord_refine((double)(-(2.0f / 3.0f) * sqf * y), P, Q);
 }
 
+// The largest root of u^3 + P u + Q = 0 (f(R) n = 1 and symmetron) by Newton's
+// method in FP32, from the cell's current value: the precision form's root and
+// the plain path's seed.  That is the root the reference's closed form returns: Cardano's
+// single real root when CC >= 0, and for CC < 0 the trigonometric form
+// -(2/3) sqrt(-3P) cos(acos(c)/3 + 2 pi/3), which lies in
+// [sqrt(-P/3), 2 sqrt(-P/3)], right of the local minimum.
+// To the right of the local minimum (3u^2 + P > 0) the cubic is convex, so
+// Newton converges to that root from any such start, quadratically with
+// eps' <= 3.3 eps^2 while 3u^2 + P >= 0.9 u^2: a step below 1e-4 u leaves an
+// error below FP32 rounding.  Returns NaN when the start is outside that region
+// or five steps do not converge; the caller then takes the FP64 closed form.
+__device__ __forceinline__ float cubic_root_newton32(float u, float P, float Q) {
+    if (!(u > 0.0f && u < 1.0e15f && fmaf(2.1f * u, u, P) > 0.0f)) return __int_as_float(0x7fffffff);
+#pragma unroll 1
+    for (int it = 0; it < 5; ++it) {
+        const float fp = fmaf(3.0f * u, u, P);
+        const float f = fmaf(fmaf(u, u, P), u, Q);
+        const float du = f * rcp_approx(fp);
+        u = u - du;
+        if (fabsf(du) <= 1.0e-4f * u) return u;
+    }
+    return __int_as_float(0x7fffffff);
+}
+
+// f(R) n = 2: the positive root of u^4 + P u + Q = 0 (Q < 0),
+// the root the reference's Ferrari closed form returns, by Newton's method in
+// FP32 from the cell's current value.  The quartic is convex with one positive
+// root; right of its minimum (4u^3 + P > 0) Newton converges from any start,
+// with eps' <= 5 eps^2 while 4u^3 + P >= 1.2 u^3.  NaN when the start is
+// unusable or five steps do not converge.
+__device__ __forceinline__ float quartic_root_newton32(float u, float P, float Q) {
+    if (!(u > 0.0f && u < 1.0e10f && fmaf(2.8f * u * u, u, P) > 0.0f)) return __int_as_float(0x7fffffff);
+#pragma unroll 1
+    for (int it = 0; it < 5; ++it) {
+        const float u2 = u * u;
+        const float fp = fmaf(4.0f * u2, u, P);
+        const float f = fmaf(fmaf(u2, u, P), u, Q);
+        const float du = f * rcp_approx(fp);
+        u = u - du;
+        if (fabsf(du) <= 1.0e-4f * u) return u;
+    }
+    return __int_as_float(0x7fffffff);
+}
+
+// FP64 root of the plain path from an FP32 seed: two chord steps, each of which
+// multiplies the relative error by ~1e-6 (see chord_refine); NaN when the seed is
+// unusable or sits near a double root.
+template <bool QUARTIC>
+__device__ __forceinline__ double refine_seed(float u0, double P, double Q) {
+    const float u2 = u0 * u0;
+    const float fp = QUARTIC ? fmaf(4.0f * u2, u0, (float)P) : fmaf(3.0f, u2, (float)P);
+    if (!(u0 > 1.0e-15f && fabsf(fp) > 3.0e-3f * (QUARTIC ? u2 * u0 : u2))) return (double)__int_as_float(0x7fffffff);
+    const double r = (double)rcp_approx(fp);
+    double u = (double)u0;
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+        const double f = QUARTIC ? fma(fma(u * u, u, P), u, Q) : fma(fma(u, u, P), u, Q);
+        u = fma(-f, r, u);
+    }
+    return u;
+}
+
+// The closed forms for the rare cells without a usable FP32 root, out of line:
+// inlined into every cell of the fused sweep they took its registers and most of
+// its code.  third: the root at P = 0.
+__device__ __noinline__ double cubic_root_cold(double P, double Q, double D1, double third) {
+    const double D0 = -3.0 * P;
+    const double CC = D1 * D1 - 4.0 * D0 * D0 * D0;
+    if (CC >= 0.0) {
+        if (fabs(P) < 1.0e-20) return third;
+        return cardano_root(P, Q, CC, D0, D1);
+    }
+    return trig_root(P, Q, D0, D1);
+}
+__device__ __noinline__ double sym_root_cold(double P, double Q) { return cubic_root_cold(P, Q, 27.0 * Q, -scbrt(Q)); }
+__device__ __noinline__ double quartic_root_cold(double P, double Q, double D20) {
+    const double Delta21 = 27.0 * P * P;
+    const double tmp1 = 0.5 * (sqrt(Delta21 * Delta21 - 4.0 * D20 * D20 * D20) + Delta21);
+    const double cr = scbrt(tmp1);
+    const double S = sqrt(cr + D20 / cr) / sqrt(12.0);
+    if (P > 1.0e-20) return -S + 0.5 * sqrt(-4.0 * S * S + P / S);
+    if (P < -1.0e-20) return S + 0.5 * sqrt(-4.0 * S * S - P / S);
+    return sqrt(sqrt(-Q));
+}
+
+
+// The plain path's cubic (quartic) root from the cell's current value: the FP32
+// Newton root refined in FP64, else the closed form.  The value is the closed form's
+// to FP64 rounding, as before, at a third of its instructions.
+template <bool QUARTIC>
+__device__ __forceinline__ double root_from(float uold, double P, double Q) {
+    const float seed = QUARTIC ? quartic_root_newton32(uold, (float)P, (float)Q)
+                               : cubic_root_newton32(uold, (float)P, (float)Q);
+    return refine_seed<QUARTIC>(seed, P, Q);
+}
+
 // ------------------------------------------------------------- f(R) -------
 // c / u in FP64: an SFU reciprocal seed of u refined by two Newton steps
 // (relative error 2^-22 -> 2^-44 -> FP64 rounding), exact division outside
@@ -350,25 +444,13 @@ __device__ __forceinline__ double div_by(double c, float u) {
     return c * r;
 }
 
+// The new value of an f(R) cell (uold: its current value)
 template <int FRN>
-__device__ __forceinline__ double fr_root(double P, const LevelConsts& k) {
-    if (FRN == 0) return 0.5 * (-P + sqrt(P * P - k.fr_Q4));
-    if (FRN == 1) {
-        const double Delta10 = -3.0 * P;
-        const double CC = k.fr_D11 * k.fr_D11 - 4.0 * Delta10 * Delta10 * Delta10;
-        if (CC >= 0.0) {
-            if (fabs(P) < 1.0e-20) return k.fr_Q2third;
-            return cardano_root(P, k.fr_Q, CC, Delta10, k.fr_D11);
-        }
-        return trig_root(P, k.fr_Q, Delta10, k.fr_D11);
-    }
-    const double Delta21 = 27.0 * P * P;
-    const double tmp1 = 0.5 * (sqrt(Delta21 * Delta21 - 4.0 * k.fr_D20 * k.fr_D20 * k.fr_D20) + Delta21);
-    const double cr = scbrt(tmp1);
-    const double S = sqrt(cr + k.fr_D20 / cr) / sqrt(12.0);
-    if (P > 1.0e-20) return -S + 0.5 * sqrt(-4.0 * S * S + P / S);
-    if (P < -1.0e-20) return S + 0.5 * sqrt(-4.0 * S * S - P / S);
-    return sqrt(sqrt(-k.fr_Q));
+__device__ __forceinline__ float fr_root(float uold, double P, const LevelConsts& k) {
+    if (FRN == 0) return (float)(0.5 * (-P + sqrt(P * P - k.fr_Q4)));
+    const double u = root_from<FRN == 2>(uold, P, k.fr_Q);
+    if (u == u) return (float)u;
+    return (float)(FRN == 1 ? cubic_root_cold(P, k.fr_Q, k.fr_D11, k.fr_Q2third) : quartic_root_cold(P, k.fr_Q, k.fr_D20));
 }
 
 __device__ __forceinline__ int lg2(int n) { return __ffs(n) - 1; }   // n is a power of two
@@ -404,7 +486,7 @@ __device__ __forceinline__ void relax_fr_cells(float* __restrict__ u, const floa
         double P = kc.fr_fct1 * (double)d[q.c] - kc.fr_Q2;
         if (!L0) P = P + kc.fr_fct2 * (double)tau[q.c];
         P = P - (double)s * (1.0 / 6.0);
-        u[q.c] = (float)fr_root<FRN>(P, kc);
+        u[q.c] = fr_root<FRN>(FRN == 0 ? 0.0f : u[q.c], P, kc);
     }
 }
 
@@ -670,15 +752,8 @@ __device__ __forceinline__ void relax_sym_cells(float* __restrict__ u, const flo
         s = s + u[q.zl];
         const double P = kc.sy_fct1 * ((double)d[q.c] + 1.0) - 1.0 + kc.sy_f3;
         const double Q = L0 ? kc.sy_f2 * (double)s : kc.sy_fct4 * (double)tau[q.c] + kc.sy_f2 * (double)s;
-        const double D0 = -3.0 * P, D1 = 27.0 * Q;
-        const double CC = D1 * D1 - 4.0 * D0 * D0 * D0;
-        double val;
-        if (CC >= 0.0) {
-            if (fabs(P) < 1.0e-20) val = -scbrt(Q);
-            else val = cardano_root(P, Q, CC, D0, D1);
-        } else {
-            val = trig_root(P, Q, D0, D1);
-        }
+        double val = root_from<false>(u[q.c], P, Q);
+        if (val != val) val = sym_root_cold(P, Q);
         u[q.c] = (float)val;
     }
 }
@@ -692,69 +767,47 @@ __global__ void k_relax_sym(float* __restrict__ u, const float* __restrict__ d, 
 // ------------------------------------------------ fused red-black sweep ----
 // One smoothing iteration (red pass, then black pass) of a 7-point model in a
 // single sweep.  A block owns an interior tile of FB_X x FB_Y cells in x-y and a
-// chunk of planes in z, and marches up the chunk keeping five planes of the
-// field (with a 2-cell halo) in a shared-memory ring.  Step m has two phases:
-//   A: red cells of plane m (tile and its 1-cell ring) and black cells of
-//      plane m-2 (tile), side by side;
-//   B: write plane m-2; plane m+2 (prefetched into registers during A)
-//      replaces plane m-3 in the ring.
-// Red(m) reads only old black values (black(m-1) comes one step later) and
+// chunk of planes in z, and marches up the chunk keeping six planes of the
+// field (with a 2-cell halo) in a shared-memory ring.  Step m updates the red
+// cells of plane m (tile and its 1-cell ring) and the black cells of plane m-2
+// (tile), and puts plane m+2 (fetched into registers at the start of the step)
+// into the slot of plane m-4.  Red(m) reads only old black values and
 // black(m-2) only new red values of planes m-3 .. m-1, so every cell gets
-// exactly the arithmetic of the two separate passes, with two barriers per
+// exactly the arithmetic of the two separate passes, with one barrier per
 // plane.  The result goes to a second buffer (blocks read halos that other
 // blocks own), so two calls per smoothing step return the field to its buffer.
-// Each interior thread updates two cells of a colour per plane, 64 apart in x.
-constexpr int FB_X = 128, FB_Y = 16, FB_PX = FB_X + 4, FB_PY = FB_Y + 4, FB_PLANE = FB_PX * FB_PY;
+//
+// A row of a plane is stored split by the parity of x (even cells, then odd
+// ones).  A thread owns four consecutive cells of a row, two of each colour,
+// which are adjacent in their half row: each neighbour direction of the two
+// cells is one 8-byte load (the x neighbours one more word), 7 loads for 2
+// cells instead of 14.  The new black values are read by nobody in this sweep,
+// and the two red cells between them are already in registers as their x
+// neighbours, so the four go straight to memory as one 16-byte store.
+//
+// What bounds it is instruction issue (ncu, precision form at 512^3: 0.71 of the
+// slots, 390 warp instructions per warp and plane, 0.37 of DRAM bandwidth); two
+// blocks of 16 warps at 64 registers, the four cells' roots side by side, do better
+// than three blocks of 21 warps at 32 registers with one root after the other.  Per
+// launch, before -> after: precision form f(R) n = 1 at 1024^3 4.37 -> 4.07 ms (0.48
+// of the measured copy bandwidth), at 512^3 0.570 -> 0.501, symmetron at 512^3 0.645
+// -> 0.517; plain path at 256^3 f(R) n = 1 0.173 -> 0.110 (whose root was a closed
+// form with exp2 and log2 seeds), n = 2 0.235 -> 0.112 (FP64 square and cube roots),
+// symmetron 0.131 -> 0.114.  Three blocks (40 registers) spill: 4.41 ms at 1024^3;
+// the densities loaded when needed instead of staged: 4.19 ms; separate barriers
+// for red cells and planes with a step of slack each: bit-identical, 4.06 against
+// 3.88 ms.
+constexpr int FB_X = 128, FB_Y = 16, FB_HALF = FB_X / 2 + 4, FB_ROW = 2 * FB_HALF, FB_ROWS = FB_Y + 4;
+constexpr int FB_PLANE = FB_ROW * FB_ROWS, FB_RING = 6;
 constexpr int FB_HALO_RED = 2 * (FB_X + 2) / 2 + FB_Y;   // red cells on the 1-cell ring per plane (146)
-constexpr int FB_INNER = FB_X / 4 * FB_Y;                // two interior updates per thread (512 threads)
-constexpr int FB_THREADS = FB_INNER + 160;               // + 5 warps for the ring
-constexpr int FB_PREF = (FB_PLANE / 2 + FB_THREADS - 1) / FB_THREADS;   // float2 prefetches per thread
-constexpr int FB_OUT4 = FB_X * FB_Y / 4;                 // float4 stores of one interior plane (512)
-constexpr int FB_SMEM = 5 * FB_PLANE * (int)sizeof(float);   // 52800 B of dynamic shared memory
-
-// Precision form (MGG_PREC_MIXED), f(R) n = 1 and symmetron: the largest root
-// of u^3 + P u + Q = 0 by Newton's method in FP32, from the cell's current
-// value.  That is the root the reference's closed form returns: Cardano's
-// single real root when CC >= 0, and for CC < 0 the trigonometric form
-// -(2/3) sqrt(-3P) cos(acos(c)/3 + 2 pi/3), which lies in
-// [sqrt(-P/3), 2 sqrt(-P/3)], right of the local minimum.
-// To the right of the local minimum (3u^2 + P > 0) the cubic is convex, so
-// Newton converges to that root from any such start, quadratically with
-// eps' <= 3.3 eps^2 while 3u^2 + P >= 0.9 u^2: a step below 1e-4 u leaves an
-// error below FP32 rounding.  Returns NaN when the start is outside that region
-// or five steps do not converge; the caller then takes the FP64 closed form.
-__device__ __forceinline__ float cubic_root_newton32(float u, float P, float Q) {
-    if (!(u > 0.0f && u < 1.0e15f && fmaf(2.1f * u, u, P) > 0.0f)) return __int_as_float(0x7fffffff);
-#pragma unroll 1
-    for (int it = 0; it < 5; ++it) {
-        const float fp = fmaf(3.0f * u, u, P);
-        const float f = fmaf(fmaf(u, u, P), u, Q);
-        const float du = f * rcp_approx(fp);
-        u = u - du;
-        if (fabsf(du) <= 1.0e-4f * u) return u;
-    }
-    return __int_as_float(0x7fffffff);
-}
-
-// Precision form, f(R) n = 2: the positive root of u^4 + P u + Q = 0 (Q < 0),
-// the root the reference's Ferrari closed form returns, by Newton's method in
-// FP32 from the cell's current value.  The quartic is convex with one positive
-// root; right of its minimum (4u^3 + P > 0) Newton converges from any start,
-// with eps' <= 5 eps^2 while 4u^3 + P >= 1.2 u^3.  NaN when the start is
-// unusable or five steps do not converge.
-__device__ __forceinline__ float quartic_root_newton32(float u, float P, float Q) {
-    if (!(u > 0.0f && u < 1.0e10f && fmaf(2.8f * u * u, u, P) > 0.0f)) return __int_as_float(0x7fffffff);
-#pragma unroll 1
-    for (int it = 0; it < 5; ++it) {
-        const float u2 = u * u;
-        const float fp = fmaf(4.0f * u2, u, P);
-        const float f = fmaf(fmaf(u2, u, P), u, Q);
-        const float du = f * rcp_approx(fp);
-        u = u - du;
-        if (fabsf(du) <= 1.0e-4f * u) return u;
-    }
-    return __int_as_float(0x7fffffff);
-}
+constexpr int FB_INNER = FB_X / 4 * FB_Y;                // four cells per thread (512 threads)
+constexpr int FB_THREADS = FB_INNER;
+// dynamic shared memory: the ring, and on the finest level (whose cells read only
+// the density beside the field) five planes of the tile's densities, 106240 B in all
+constexpr int FB_DSLOTS = 5;
+constexpr int fb_smem(bool l0) { return FB_RING * FB_PLANE * 4 + (l0 ? FB_DSLOTS * FB_THREADS * 16 : 0); }
+// word of cell (x, y), relative to the tile (x, y >= -2), in a plane
+__device__ __forceinline__ int fb_at(int x, int y) { return (y + 2) * FB_ROW + (x & 1) * FB_HALF + ((x + 4) >> 1); }
 
 // One cell of the precision-form f(R) sweep: P in FP32 from the FP32
 // neighbour sum, then the root in FP32 -- n = 0: the larger root of
@@ -779,7 +832,9 @@ __device__ __forceinline__ float fr_update_mixed(float s, float uold, float dvf,
     double Pd = kc.fr_fct1 * (double)dvf - kc.fr_Q2;
     if (!L0) Pd = Pd + kc.fr_fct2 * (double)tvf;
     Pd = Pd - (double)s * (1.0 / 6.0);
-    return (float)fr_root<FRN>(Pd, kc);
+    if (FRN == 1) return (float)cubic_root_cold(Pd, kc.fr_Q, kc.fr_D11, kc.fr_Q2third);
+    if (FRN == 2) return (float)quartic_root_cold(Pd, kc.fr_Q, kc.fr_D20);
+    return fr_root<0>(0.0f, Pd, kc);
 }
 
 // One cell of a 7-point red-black sweep from its six neighbours (the reference's
@@ -800,7 +855,7 @@ __device__ __forceinline__ float cell_update(float nxu, float nxl, float nyu, fl
         double P = kc.fr_fct1 * dval - kc.fr_Q2;
         if (!L0) P = P + kc.fr_fct2 * tval;
         P = P - (double)s * (1.0 / 6.0);
-        return (float)fr_root<FRN>(P, kc);
+        return fr_root<FRN>(c0, P, kc);
     } else {
         float s = nxu;
         s = s + nxl;
@@ -813,108 +868,316 @@ __device__ __forceinline__ float cell_update(float nxu, float nxl, float nyu, fl
             const float Qf = L0 ? kc.f_sy_f2 * s : fmaf(kc.f_sy_fct4, tvf, kc.f_sy_f2 * s);
             const float u = cubic_root_newton32(c0, Pf, Qf);
             if (u == u) return u;
+            return (float)sym_root_cold(kc.sy_fct1 * (dval + 1.0) - 1.0 + kc.sy_f3,
+                                        L0 ? kc.sy_f2 * (double)s : kc.sy_fct4 * tval + kc.sy_f2 * (double)s);
         }
         const double P = kc.sy_fct1 * (dval + 1.0) - 1.0 + kc.sy_f3;
         const double Q = L0 ? kc.sy_f2 * (double)s : kc.sy_fct4 * tval + kc.sy_f2 * (double)s;
-        const double D0 = -3.0 * P, D1 = 27.0 * Q;
-        const double CC = D1 * D1 - 4.0 * D0 * D0 * D0;
-        if (CC >= 0.0) {
-            if (fabs(P) < 1.0e-20) return (float)(-scbrt(Q));
-            return (float)cardano_root(P, Q, CC, D0, D1);
-        }
-        return (float)trig_root(P, Q, D0, D1);
+        const double u = root_from<false>(c0, P, Q);
+        return (float)(u == u ? u : sym_root_cold(P, Q));
     }
 }
 
-template <int MODEL, int FRN, bool L0, bool MIX>
-__device__ __forceinline__ float fused_update(const float* __restrict__ S0, const float* __restrict__ Sm,
-                                              const float* __restrict__ Sp, int p, float dvf, float tvf,
-                                              const LevelConsts& kc) {
-    return cell_update<MODEL, FRN, L0, MIX>(S0[p + 1], S0[p - 1], S0[p + FB_PX], S0[p - FB_PX], Sp[p], Sm[p],
-                                            MIX ? S0[p] : 0.0f, dvf, tvf, kc);
+// f(R) n = 0: the larger root of u^2 + P u + Q in closed form
+template <bool L0, bool MIX>
+__device__ __forceinline__ float cell_root0(float s, float dvf, float tvf, const LevelConsts& kc) {
+    if (MIX) return fr_update_mixed<0, L0>(s, 0.0f, dvf, tvf, kc);
+    double P = kc.fr_fct1 * (double)dvf - kc.fr_Q2;
+    if (!L0) P = P + kc.fr_fct2 * (double)tvf;
+    P = P - (double)s * (1.0 / 6.0);
+    return fr_root<0>(0.0f, P, kc);
 }
 
-// f(R) with n = 1 fits 32 registers: three blocks (63 warps) per SM
-// three blocks per SM (32 registers) for the f(R) n = 1 smoother; on the coarse
-// levels (which also load tau) the precision form at two blocks (40 registers)
-// measured 1-2 % faster
-template <int MODEL, int FRN, bool L0, bool MIX>
-constexpr int fb_min_blocks() { return (MODEL == MGG_MODEL_FR && FRN == 1 && (L0 || !MIX)) ? 3 : 2; }
+// Two FP32 values in one register pair: packed operations, lane by lane the scalar ones.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n"
+        " fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 x, x, y;\n"
+        " mov.b64 {%0, %1}, x;\n}" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n"
+        " mov.b64 {%0, %1}, x;\n}" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+// Two cells of one colour in one row: the Real*4 neighbour sum s (of the powers
+// for f(R)), density, tau and the cells' current values (the Newton start).
+struct Pair {
+    float2 s, d, t, u;
+};
+
+// From the planes below, at and above (Sm, S0, Sp; a: the pair's words, b: the
+// words of the other parity of x, xs: the outer x neighbour -- see the layout
+// above); odd: the pair sits at odd x.  The x neighbours between the cells are
+// handed back in nb.  Neighbours in the reference's order x+, x-, y+, y-, z+, z-.
+template <int MODEL, int FRN>
+__device__ __forceinline__ Pair load_pair(const float* __restrict__ Sm, const float* __restrict__ S0,
+                                          const float* __restrict__ Sp, int a, int b, int xs, bool odd, float4 d4,
+                                          float4 t4, float2& nb) {
+    auto ld2 = [](const float* q) { return *reinterpret_cast<const float2*>(q); };
+    nb = ld2(S0 + b);
+    const float o = S0[xs];
+    const float2 yu = ld2(S0 + a + FB_ROW), yl = ld2(S0 + a - FB_ROW), zu = ld2(Sp + a), zl = ld2(Sm + a);
+    const float2 xu = odd ? make_float2(nb.y, o) : nb, xl = odd ? nb : make_float2(o, nb.x);
+    Pair c;
+    if (MODEL == MGG_MODEL_FR && FRN == 1) {
+        c.s = fma2(zl, zl, fma2(zu, zu, fma2(yl, yl, fma2(yu, yu, fma2(xl, xl, mul2(xu, xu))))));
+    } else if (MODEL == MGG_MODEL_FR && FRN == 2) {
+        auto cube = [](float2 v, float2 w) { return fma2(mul2(v, v), v, w); };
+        c.s = cube(zl, cube(zu, cube(yl, cube(yu, cube(xl, mul2(mul2(xu, xu), xu))))));
+    } else {
+        c.s = add2(add2(add2(add2(add2(xu, xl), yu), yl), zu), zl);
+    }
+    c.d = odd ? make_float2(d4.y, d4.w) : make_float2(d4.x, d4.z);
+    c.t = odd ? make_float2(t4.y, t4.w) : make_float2(t4.x, t4.z);
+    c.u = ld2(S0 + a);
+    return c;
+}
+
+// Newton's method in FP32 from the cells' current values on u^3 + P u + Q (quartic:
+// u^4 + P u + Q), all NP pairs in step, so that each iteration's chain (two or
+// three multiply-adds, a reciprocal) runs for 2 NP cells side by side.  Each cell
+// gets the steps of cubic_root_newton32 / quartic_root_newton32 and stops where they
+// do, so its value does not depend on the cells beside it.  NaN where the start is
+// unusable or five steps do not converge.
+template <bool QUARTIC, int NP>
+__device__ __forceinline__ void newton_pairs(float2 (&u)[NP], const float2 (&P)[NP], const float2 (&Q)[NP]) {
+    const float nan = __int_as_float(0x7fffffff);
+    auto start = [&](float v, float p) {
+        return QUARTIC ? v > 0.0f && v < 1.0e10f && fmaf(2.8f * v * v, v, p) > 0.0f
+                       : v > 0.0f && v < 1.0e15f && fmaf(2.1f * v, v, p) > 0.0f;
+    };
+    bool ax[NP], ay[NP], more = false;   // cells still under way
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        ax[i] = start(u[i].x, P[i].x);
+        ay[i] = start(u[i].y, P[i].y);
+        if (!ax[i]) u[i].x = nan;
+        if (!ay[i]) u[i].y = nan;
+        more |= ax[i] || ay[i];
+    }
+#pragma unroll 1
+    for (int it = 0; it < 5 && more; ++it) {
+        more = false;
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            float2 f, fp;
+            if (QUARTIC) {
+                const float2 u2 = mul2(u[i], u[i]);
+                f = fma2(fma2(u2, u[i], P[i]), u[i], Q[i]);
+                fp = fma2(mul2(both(4.0f), u2), u[i], P[i]);
+            } else {
+                f = fma2(fma2(u[i], u[i], P[i]), u[i], Q[i]);
+                fp = fma2(mul2(both(3.0f), u[i]), u[i], P[i]);
+            }
+            const float2 du = mul2(f, make_float2(ax[i] ? -rcp_approx(fp.x) : 0.0f, ay[i] ? -rcp_approx(fp.y) : 0.0f));
+            u[i] = add2(u[i], du);
+            ax[i] = ax[i] && fabsf(du.x) > 1.0e-4f * u[i].x;
+            ay[i] = ay[i] && fabsf(du.y) > 1.0e-4f * u[i].y;
+            more |= ax[i] || ay[i];
+        }
+    }
+    if (more) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            if (ax[i]) u[i].x = nan;
+            if (ay[i]) u[i].y = nan;
+        }
+    }
+}
+
+// The new values of NP pairs (side by side: the root's chain is long and a step
+// has two independent pairs).  A cell without a usable root takes the FP64 closed
+// form out of line.
+template <int MODEL, int FRN, bool L0, bool MIX, int NP>
+__device__ __forceinline__ void update_pairs(Pair (&c)[NP], const LevelConsts& kc) {
+    constexpr bool FR = MODEL == MGG_MODEL_FR, QUARTIC = FR && FRN == 2;
+    if constexpr (FR && FRN == 0) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            c[i].u.x = cell_root0<L0, MIX>(c[i].s.x, c[i].d.x, c[i].t.x, kc);
+            c[i].u.y = cell_root0<L0, MIX>(c[i].s.y, c[i].d.y, c[i].t.y, kc);
+        }
+        return;
+    }
+    auto P64 = [&](float s, float d, float t) {
+        if (!FR) return kc.sy_fct1 * ((double)d + 1.0) - 1.0 + kc.sy_f3;
+        double P = kc.fr_fct1 * (double)d - kc.fr_Q2;
+        if (!L0) P = P + kc.fr_fct2 * (double)t;
+        return P - (double)s * (1.0 / 6.0);
+    };
+    auto Q64 = [&](float s, float t) {
+        if (FR) return kc.fr_Q;
+        return L0 ? kc.sy_f2 * (double)s : kc.sy_fct4 * (double)t + kc.sy_f2 * (double)s;
+    };
+    auto cold = [&](float s, float d, float t) {
+        const double P = P64(s, d, t);
+        if (!FR) return sym_root_cold(P, Q64(s, t));
+        if (QUARTIC) return quartic_root_cold(P, kc.fr_Q, kc.fr_D20);
+        return cubic_root_cold(P, kc.fr_Q, kc.fr_D11, kc.fr_Q2third);
+    };
+    float2 P[NP], Q[NP], u[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        if constexpr (!MIX) {
+            P[i] = make_float2((float)P64(c[i].s.x, c[i].d.x, c[i].t.x), (float)P64(c[i].s.y, c[i].d.y, c[i].t.y));
+            Q[i] = FR ? both(kc.f_Q) : make_float2((float)Q64(c[i].s.x, c[i].t.x), (float)Q64(c[i].s.y, c[i].t.y));
+        } else if constexpr (FR) {
+            P[i] = fma2(both(kc.f_fct1), c[i].d, both(kc.f_mQ2));
+            if (!L0) P[i] = fma2(both(kc.f_fct2), c[i].t, P[i]);
+            P[i] = fma2(c[i].s, both(-1.0f / 6.0f), P[i]);
+            Q[i] = both(kc.f_Q);
+        } else {
+            P[i] = add2(fma2(both(kc.f_sy_fct1), add2(c[i].d, both(1.0f)), both(-1.0f)), both(kc.f_sy_f3));
+            Q[i] = mul2(both(kc.f_sy_f2), c[i].s);
+            if (!L0) Q[i] = fma2(both(kc.f_sy_fct4), c[i].t, Q[i]);
+        }
+        u[i] = c[i].u;
+    }
+    newton_pairs<QUARTIC, NP>(u, P, Q);
+    if constexpr (!MIX) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            u[i].x = (float)refine_seed<QUARTIC>(u[i].x, P64(c[i].s.x, c[i].d.x, c[i].t.x), Q64(c[i].s.x, c[i].t.x));
+            u[i].y = (float)refine_seed<QUARTIC>(u[i].y, P64(c[i].s.y, c[i].d.y, c[i].t.y), Q64(c[i].s.y, c[i].t.y));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        if (u[i].x != u[i].x) u[i].x = (float)cold(c[i].s.x, c[i].d.x, c[i].t.x);
+        if (u[i].y != u[i].y) u[i].y = (float)cold(c[i].s.y, c[i].d.y, c[i].t.y);
+        c[i].u = u[i];
+    }
+}
 
 template <int MODEL, int FRN, bool L0, bool MIX = false>
-__global__ void __launch_bounds__(FB_THREADS, fb_min_blocks<MODEL, FRN, L0, MIX>()) k_smooth_fused(
+__global__ void __launch_bounds__(FB_THREADS, 2) k_smooth_fused(
     const float* __restrict__ uin, float* __restrict__ uout, const float* __restrict__ d, const float* __restrict__ tau,
     int n, int cz, LevelConsts kc) {
-    extern __shared__ __align__(16) float S[];   // FB_SMEM bytes: five padded planes
+    extern __shared__ __align__(16) float S[];   // fb_smem(L0) bytes
     const int x0 = blockIdx.x * FB_X, y0 = blockIdx.y * FB_Y, kbeg = blockIdx.z * cz, kend = kbeg + cz;
     const int nm = n - 1;
     const int plane = n * n;   // offsets fit 32 bits: n^3 <= 2^30
-    const int tid = threadIdx.x;
-    // x-y offsets (periodic) of this thread's float2 pairs of a padded plane; pairs
-    // start at even x, so they never straddle the periodic wrap
-    int pxy[FB_PREF], sxy[FB_PREF];
-#pragma unroll
-    for (int i = 0; i < FB_PREF; ++i) {
-        const int e = min(tid + i * FB_THREADS, FB_PLANE / 2 - 1);
-        const int yy = e / (FB_PX / 2), xx = 2 * (e - yy * (FB_PX / 2));
-        pxy[i] = ((x0 + xx - 2) & nm) + n * ((y0 + yy - 2) & nm);
-        sxy[i] = yy * FB_PX + xx;
-    }
-    // planes kbeg-2 .. kbeg go to ring slots 2, 3, 4 (planes m-1, m, m+1 of the
-    // first step m = kbeg - 1)
-    for (int z = kbeg - 2; z <= kbeg; ++z) {
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    // Loads of a plane: every thread its own four cells; warps 0..3 also the rows y = -2, -1, 16,
+    // 17, and warps 4, 5 the two cells on either side of the 20 rows, as pairs that start at even
+    // x and never straddle the periodic wrap.  Warps 6..10 also update the ring's red cells.
+    const int gxy = x0 + 4 * lane + n * (y0 + w);
+    const int p0 = fb_at(4 * lane, w);
+    const bool hrow = w < 4;
+    const int e = tid - 128;
+    const bool edge = e >= 0 && e < 2 * FB_ROWS;
+    const int hy = hrow ? (w < 2 ? w - 2 : FB_Y + w - 2) : (e >> 1) - 2;
+    const int hx = hrow ? 4 * lane : (e & 1 ? FB_X : -2);
+    const int hsrc = ((x0 + hx) & nm) + n * ((y0 + hy) & nm), hdst = hrow || edge ? fb_at(hx, hy) : 0;
+    const int h = tid - 192;   // ring cell
+    auto fetch_plane = [&](int z, float4& v, float4& v2) {
         const float* uz = uin + (z & nm) * plane;
-        float* Sz = S + (z - kbeg + 4) * FB_PLANE;
-#pragma unroll
-        for (int i = 0; i < FB_PREF; ++i)
-            if (tid + i * FB_THREADS < FB_PLANE / 2)
-                *reinterpret_cast<float2*>(Sz + sxy[i]) = __ldg(reinterpret_cast<const float2*>(uz + pxy[i]));
+        v = __ldg(reinterpret_cast<const float4*>(uz + gxy));
+        if (hrow) {
+            v2 = __ldg(reinterpret_cast<const float4*>(uz + hsrc));
+        } else if (edge) {
+            const float2 q = __ldg(reinterpret_cast<const float2*>(uz + hsrc));
+            v2.x = q.x;
+            v2.y = q.y;
+        }
+    };
+    auto store_plane = [&](float* Sz, const float4& v, const float4& v2) {
+        *reinterpret_cast<float2*>(Sz + p0) = make_float2(v.x, v.z);
+        *reinterpret_cast<float2*>(Sz + p0 + FB_HALF) = make_float2(v.y, v.w);
+        if (hrow) {
+            *reinterpret_cast<float2*>(Sz + hdst) = make_float2(v2.x, v2.z);
+            *reinterpret_cast<float2*>(Sz + hdst + FB_HALF) = make_float2(v2.y, v2.w);
+        } else if (edge) {
+            Sz[hdst] = v2.x;
+            Sz[hdst + FB_HALF] = v2.y;
+        }
+    };
+    float4 pre, pre2;
+    // Finest level: each thread copies the densities of its own four cells two planes ahead
+    // (asynchronously, read back by itself: red at step m, black at m+2), so that no update
+    // waits for them; slot dq holds plane m.
+    float4* const DS = reinterpret_cast<float4*>(S + FB_RING * FB_PLANE) + tid;
+    auto stage = [&](int z, int slot) {
+        if (z <= kend) {
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(DS + slot * FB_THREADS);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(d + (z & nm) * plane + gxy) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int dq = 0;
+    if (L0) {
+        stage(kbeg - 1, 0);
+        stage(kbeg, 1);
     }
-    const bool inner = tid < FB_INNER;
-    const int w = tid >> 5, lane = tid & 31;
-    // interior cells of this thread: x = 2 lane + parity (+ 64), y = w (no wrap inside the tile)
-    const int ixy = x0 + 2 * lane + n * (y0 + w);
-    const int ip = (w + 2) * FB_PX + 2 * lane + 2;
-    const int h = tid - FB_INNER;   // ring cell index of warps 16..20
-    // this thread's float4 of the interior plane for the write-out
-    const int oy = tid >> 5, ox = 4 * (tid & 31);
-    const int oxy = (x0 + ox) + n * (y0 + oy), osm = (oy + 2) * FB_PX + ox + 2;
-    float2 pre[FB_PREF];
-    // One step m with the ring slots (float offsets into S) of planes m-3, m-2,
-    // m-1, m, m+1: (j + 0..4) mod 5 planes with j = m - kbeg + 1.  The
-    // precision-form sweeps run five steps per loop iteration and pass the slots
-    // as compile-time constants; the plain sweeps (whose FP64 closed-form root is
-    // the main path, five copies of which slowed the whole run) keep one step per
-    // iteration and rotate the slots in registers.
-    auto step = [&](int m, auto oE, auto oA, auto oB, auto oC, auto oD) {
+    // planes kbeg-2 .. kbeg go to ring slots 3, 4, 5 (planes m-1, m, m+1 of the
+    // first step m = kbeg - 1; the slots of step m are those of planes m-4 .. m+1)
+#pragma unroll 1
+    for (int z = kbeg - 2; z <= kbeg; ++z) {
+        fetch_plane(z, pre, pre2);
+        store_plane(S + (z - kbeg + 5) * FB_PLANE, pre, pre2);
+    }
+    // One step m with the ring slots (float offsets into S) of planes m-4 .. m+1:
+    // (j + 0..5) mod 6 planes with j = m - kbeg + 1.
+    auto step = [&](int m, int oF, int oE, int oA, int oB, int oC, int oD) {
         const bool fetch = m + 2 <= kend + 1;
-        if (fetch) {
-            const float* uz = uin + ((m + 2) & nm) * plane;
-#pragma unroll
-            for (int i = 0; i < FB_PREF; ++i)
-                if (tid + i * FB_THREADS < FB_PLANE / 2) pre[i] = __ldg(reinterpret_cast<const float2*>(uz + pxy[i]));
+        if (fetch) fetch_plane(m + 2, pre, pre2);
+        const bool red = m <= kend, black = m >= kbeg + 2;
+        const int gr = (m & nm) * plane + gxy, gb = ((m - 2) & nm) * plane + gxy;
+        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 dr, db, tr = z4, tb = z4;
+        if (L0) {
+            stage(m + 2, dq >= 3 ? dq - 3 : dq + 2);
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            dr = DS[dq * FB_THREADS];
+            db = DS[(dq >= 2 ? dq - 2 : dq + 3) * FB_THREADS];
+            dq = dq == 4 ? 0 : dq + 1;
+        } else {
+            dr = __ldg(reinterpret_cast<const float4*>(d + gr));
+            tr = __ldg(reinterpret_cast<const float4*>(tau + gr));
+            db = __ldg(reinterpret_cast<const float4*>(d + gb));
+            tb = __ldg(reinterpret_cast<const float4*>(tau + gb));
         }
         __syncthreads();
-        // phase A
-        const bool black = m >= kbeg + 2;   // black cells of plane m-2 (its last red neighbour came at m-1)
-        if (inner) {
-            if (m <= kend) {   // red cells of plane m: (x0 + x + y0 + y + m) even, x0 even
-                const int par = (y0 + w + m) & 1;
-                const int g = (m & nm) * plane + ixy + par, p = ip + par;
-                const float dv0 = __ldg(d + g), dv1 = __ldg(d + g + 64);
-                const float tv0 = L0 ? 0.f : __ldg(tau + g), tv1 = L0 ? 0.f : __ldg(tau + g + 64);
-                S[oC + p] = fused_update<MODEL, FRN, L0, MIX>(S + oC, S + oB, S + oD, p, dv0, tv0, kc);
-                S[oC + p + 64] = fused_update<MODEL, FRN, L0, MIX>(S + oC, S + oB, S + oD, p + 64, dv1, tv1, kc);
-            }
-            if (black) {       // black cells of plane m-2: (x + y + z) odd
-                const int par = (y0 + w + m - 1) & 1;
-                const int g = ((m - 2) & nm) * plane + ixy + par, p = ip + par;
-                const float dv0 = __ldg(d + g), dv1 = __ldg(d + g + 64);
-                const float tv0 = L0 ? 0.f : __ldg(tau + g), tv1 = L0 ? 0.f : __ldg(tau + g + 64);
-                S[oA + p] = fused_update<MODEL, FRN, L0, MIX>(S + oA, S + oE, S + oB, p, dv0, tv0, kc);
-                S[oA + p + 64] = fused_update<MODEL, FRN, L0, MIX>(S + oA, S + oE, S + oB, p + 64, dv1, tv1, kc);
-            }
-        } else if (h < FB_HALO_RED && m <= kend) {
+        const bool odd = (y0 + w + m) & 1;   // red cells of plane m in this row: x odd
+        const int a = odd ? p0 + FB_HALF : p0, b = odd ? p0 : p0 + FB_HALF;
+        // red cells of plane m ((x + y + z) even) and black cells of plane m-2 (its last red
+        // neighbour came at m-1) side by side
+        float2 nb;
+        auto red_pair = [&] {
+            float2 nr;
+            return load_pair<MODEL, FRN>(S + oB, S + oC, S + oD, a, b, odd ? b + 2 : b - 1, odd, dr, tr, nr);
+        };
+        auto black_pair = [&] {
+            return load_pair<MODEL, FRN>(S + oE, S + oA, S + oB, b, a, odd ? a - 1 : a + 2, !odd, db, tb, nb);
+        };
+        auto put_red = [&](float2 r) { *reinterpret_cast<float2*>(S + oC + a) = r; };
+        auto put_black = [&](float2 r) {
+            *reinterpret_cast<float4*>(uout + gb) = odd ? make_float4(r.x, nb.x, r.y, nb.y)
+                                                        : make_float4(nb.x, r.x, nb.y, r.y);
+        };
+        if (red && black) {
+            Pair c[2] = {red_pair(), black_pair()};
+            update_pairs<MODEL, FRN, L0, MIX, 2>(c, kc);
+            put_red(c[0].u);
+            put_black(c[1].u);
+        } else {   // the first three steps of a chunk (red only), the last (black only)
+            Pair c[1] = {red ? red_pair() : black_pair()};
+            update_pairs<MODEL, FRN, L0, MIX, 1>(c, kc);
+            if (red) put_red(c[0].u);
+            else put_black(c[0].u);
+        }
+        if (h >= 0 && h < FB_HALO_RED && m <= kend) {
             int x, y;
             if (h < FB_X + 2) {               // rows y = -1 and y = FB_Y
                 const int r = h / ((FB_X + 2) / 2), col = h - r * ((FB_X + 2) / 2);
@@ -924,52 +1187,24 @@ __global__ void __launch_bounds__(FB_THREADS, fb_min_blocks<MODEL, FRN, L0, MIX>
                 y = h - (FB_X + 2);
                 x = ((y0 + y + m) & 1) ? -1 : FB_X;
             }
-            const int p = (y + 2) * FB_PX + (x + 2);
+            const int p = fb_at(x, y), pu = fb_at(x + 1, y), pl = fb_at(x - 1, y);
             const int g = (m & nm) * plane + ((x0 + x) & nm) + n * ((y0 + y) & nm);
             const float dv = __ldg(d + g), tv = L0 ? 0.f : __ldg(tau + g);
-            S[oC + p] = fused_update<MODEL, FRN, L0, MIX>(S + oC, S + oB, S + oD, p, dv, tv, kc);
+            S[oC + p] = cell_update<MODEL, FRN, L0, MIX>(S[oC + pu], S[oC + pl], S[oC + p + FB_ROW], S[oC + p - FB_ROW],
+                                                         S[oD + p], S[oB + p], S[oC + p], dv, tv, kc);
         }
-        __syncthreads();
-        // phase B
-        if (black && tid < FB_OUT4) {
-            const float2 a = *reinterpret_cast<const float2*>(S + oA + osm);
-            const float2 b = *reinterpret_cast<const float2*>(S + oA + osm + 2);
-            *reinterpret_cast<float4*>(uout + ((m - 2) & nm) * plane + oxy) = make_float4(a.x, a.y, b.x, b.y);
-        }
-        if (fetch) {   // plane m+2 goes to the slot of plane m-3, last read by black(m-2)
-#pragma unroll
-            for (int i = 0; i < FB_PREF; ++i)
-                if (tid + i * FB_THREADS < FB_PLANE / 2) *reinterpret_cast<float2*>(S + oE + sxy[i]) = pre[i];
-        }
+        if (fetch) store_plane(S + oF, pre, pre2);   // plane m+2 in the slot of plane m-4, last read in step m-1
     };
-    if constexpr (MIX) {
-        using S0 = std::integral_constant<int, 0>;
-        using S1 = std::integral_constant<int, FB_PLANE>;
-        using S2 = std::integral_constant<int, 2 * FB_PLANE>;
-        using S3 = std::integral_constant<int, 3 * FB_PLANE>;
-        using S4 = std::integral_constant<int, 4 * FB_PLANE>;
-        for (int m = kbeg - 1; m <= kend + 1; m += 5) {
-            step(m, S0{}, S1{}, S2{}, S3{}, S4{});
-            if (m + 1 > kend + 1) break;
-            step(m + 1, S1{}, S2{}, S3{}, S4{}, S0{});
-            if (m + 2 > kend + 1) break;
-            step(m + 2, S2{}, S3{}, S4{}, S0{}, S1{});
-            if (m + 3 > kend + 1) break;
-            step(m + 3, S3{}, S4{}, S0{}, S1{}, S2{});
-            if (m + 4 > kend + 1) break;
-            step(m + 4, S4{}, S0{}, S1{}, S2{}, S3{});
-        }
-    } else {
-        int oE = 0, oA = FB_PLANE, oB = 2 * FB_PLANE, oC = 3 * FB_PLANE, oD = 4 * FB_PLANE;
-        for (int m = kbeg - 1; m <= kend + 1; ++m) {
-            step(m, oE, oA, oB, oC, oD);
-            const int t = oE;
-            oE = oA;
-            oA = oB;
-            oB = oC;
-            oC = oD;
-            oD = t;
-        }
+    int oF = 0, oE = FB_PLANE, oA = 2 * FB_PLANE, oB = 3 * FB_PLANE, oC = 4 * FB_PLANE, oD = 5 * FB_PLANE;
+    for (int m = kbeg - 1; m <= kend + 1; ++m) {
+        step(m, oF, oE, oA, oB, oC, oD);
+        const int t = oF;
+        oF = oE;
+        oE = oA;
+        oA = oB;
+        oB = oC;
+        oC = oD;
+        oD = t;
     }
 }
 
@@ -1952,26 +2187,39 @@ int tune_chunk(Ctx& c, int kind, int n, int variant, int dflt, const std::vector
 }
 
 // ---------------------------------------------------- small levels --------
-// The cycle below a level of at most 16^3 cells (MGG_COARSE_N sets the size;
+// The cycle below a level of at most 16^3 cells (MGG_COARSE_N lowers the size;
 // 0 turns it off) in one launch of one block: the host lists the level
 // operations in the order vcycle / fcycle / wcycle issue them (the colour
 // sweeps of the smoothing, the residual, the restriction, the FAS right-hand
 // side, the correction), and the block makes one pass over the level's cells
 // per operation with the per-cell code of the separate kernels, a block
-// barrier between passes.  Those levels are a few thousand cells; as separate
-// launches they cost tens of launch latencies per cycle and left the GPU idle.
-constexpr int CC_T = 512, CC_MAXOPS = 384, CC_MAXLEV = 6;
+// barrier between passes.  All of those levels' arrays (131 KB from 16^3 down)
+// live in shared memory: the passes are a few hundred to two thousand cells,
+// bound by latency, and each used to wait for L2 twice.
+constexpr int CC_T = 1024, CC_MAXOPS = 384, CC_MAXLEV = 4, CC_MAXN = 16;
+constexpr int CC_CELLS = 4096 + 512 + 64 + 8, CC_SMEM = 7 * CC_CELLS * (int)sizeof(float);
 enum : uint8_t { CO_RED = 0, CO_BLACK = 1, CO_RESID, CO_RESTRICT, CO_RHS, CO_PROLONG };
+struct CoarseArgs {
+    int nops, n;                             // n: cells per edge of level 0 (of the list)
+    uint8_t op[CC_MAXOPS], lev[CC_MAXOPS];   // lev: level index relative to the first
+    float* u;                                // the first level's field (in and out), density and right-hand side
+    const float *d, *tau;
+    LevelConsts K[CC_MAXLEV];
+};
 struct CoarseLev {
     int n;
     float *u, *d, *tau, *res, *rr, *ru, *snap;
 };
-struct CoarseArgs {
-    int nops;
-    uint8_t op[CC_MAXOPS], lev[CC_MAXOPS];   // lev: level index relative to L[0]
-    CoarseLev L[CC_MAXLEV];
-    LevelConsts K[CC_MAXLEV];
-};
+// level l (of n >> l cells per edge) in shared memory
+__device__ __forceinline__ CoarseLev coarse_level(float* sm, int n, int l) {
+    float* p = sm;
+    for (int i = 0; i < l; ++i) {
+        const int m = n >> i;
+        p += 7 * m * m * m;
+    }
+    const int m = n >> l, m3 = m * m * m;
+    return CoarseLev{m, p, p + m3, p + 2 * m3, p + 3 * m3, p + 4 * m3, p + 5 * m3, p + 6 * m3};
+}
 
 // one colour sweep of a level > 0 (as Solver::relax below the marching sizes)
 template <int MODEL, int FRN>
@@ -1993,32 +2241,44 @@ __device__ __forceinline__ void coarse_relax(const CoarseLev& L, const LevelCons
 
 template <int MODEL, int FRN>
 __global__ void __launch_bounds__(CC_T) k_coarse_cycle(const __grid_constant__ CoarseArgs a) {
-    const uint32_t t = threadIdx.x, st = blockDim.x;
+    extern __shared__ __align__(16) float sm[];
+    const uint32_t t = threadIdx.x, st = CC_T;
+    const int n3 = a.n * a.n * a.n;
+    {
+        const CoarseLev L = coarse_level(sm, a.n, 0);
+        for (int e = t; e < n3; e += st) {
+            L.u[e] = a.u[e];
+            L.d[e] = a.d[e];
+            L.tau[e] = a.tau[e];
+        }
+    }
+    __syncthreads();
     for (int o = 0; o < a.nops; ++o) {
         const int l = a.lev[o], op = a.op[o];
-        const CoarseLev& L = a.L[l];
+        const CoarseLev L = coarse_level(sm, a.n, l);
         if (op <= CO_BLACK) {
             coarse_relax<MODEL, FRN>(L, a.K[l], op, t, st);
         } else if (op == CO_RESID) {
             resid_cells<MODEL, FRN, false>(L.u, L.d, L.tau, L.res, L.n, a.K[l], t, st);
         } else if (op == CO_RESTRICT) {   // level l -> l + 1
-            const CoarseLev& C = a.L[l + 1];
+            const CoarseLev C = coarse_level(sm, a.n, l + 1);
             restrict_cells(L.res, L.u, L.d, C.n, C.rr, C.ru, C.u, C.d, t, st);
         } else if (op == CO_RHS) {
             rhs_cells<MODEL, FRN>(L.ru, L.d, L.rr, L.tau, L.n, a.K[l], t, st);
         } else {   // CO_PROLONG: correct level l from level l + 1
-            const CoarseLev& C = a.L[l + 1];
+            const CoarseLev C = coarse_level(sm, a.n, l + 1);
             prolong_cells(L.u, C.u, C.ru, L.n, MODEL, a.K[l + 1].phibar, a.K[l + 1].ctl2, t, st);
         }
         __syncthreads();
     }
+    for (int e = t; e < n3; e += st) a.u[e] = sm[e];   // the first level's field starts the shared memory
 }
 
 // size limit of the one-block cycle (cells per edge)
 int coarse_max_n() {
     static const int v = [] {
         const char* e = std::getenv("MGG_COARSE_N");
-        return e ? std::atoi(e) : 16;
+        return e ? std::min(std::atoi(e), CC_MAXN) : CC_MAXN;
     }();
     return v;
 }
@@ -2112,8 +2372,8 @@ struct Solver {
         const float* tau = l > 0 ? c.lev[l].tau : nullptr;
         ProfScope ps(c, profile ? (l == 0 ? K_MG_SMOOTH0 : K_MG_SMOOTH) : -1,
                      12.0 * (double)n * n * n + (l > 0 ? 4.0 * (double)n * n * n : 0.0));
-#define FUSED(M, F, L0) k_smooth_fused<M, F, L0><<<grid, FB_THREADS, FB_SMEM, c.stream>>>(uin, uout, d, tau, n, cz, k)
-#define FUSEDX(M, F, L0) k_smooth_fused<M, F, L0, true><<<grid, FB_THREADS, FB_SMEM, c.stream>>>(uin, uout, d, tau, n, cz, k)
+#define FUSED(M, F, L0) k_smooth_fused<M, F, L0><<<grid, FB_THREADS, fb_smem(L0), c.stream>>>(uin, uout, d, tau, n, cz, k)
+#define FUSEDX(M, F, L0) k_smooth_fused<M, F, L0, true><<<grid, FB_THREADS, fb_smem(L0), c.stream>>>(uin, uout, d, tau, n, cz, k)
         if (model == MGG_MODEL_FR && c.cfg.precision == MGG_PREC_MIXED) {
             if (l == 0) { if (frn == 0) FUSEDX(MGG_MODEL_FR, 0, true); else if (frn == 1) FUSEDX(MGG_MODEL_FR, 1, true); else FUSEDX(MGG_MODEL_FR, 2, true); }
             else { if (frn == 0) FUSEDX(MGG_MODEL_FR, 0, false); else if (frn == 1) FUSEDX(MGG_MODEL_FR, 1, false); else FUSEDX(MGG_MODEL_FR, 2, false); }
@@ -2393,14 +2653,17 @@ struct Solver {
         emit_cycle(o, l, type);
         if (!o.ok) return false;
         double cells = 0.0;
+        a.n = n;
+        a.u = c.lev[l].u;
+        a.d = c.lev[l].d;
+        a.tau = c.lev[l].tau;
         for (int q = l; q <= c.levelmax && q - l < CC_MAXLEV; ++q) {
             const Level& V = c.lev[q];
-            a.L[q - l] = CoarseLev{V.n, V.u, V.d, V.tau, V.res, V.rr, V.ru, V.snap};
             a.K[q - l] = make_consts(c, q);
             cells += (double)V.n * V.n * V.n;
         }
         ProfScope ps(c, K_MG_COARSE, 16.0 * 4.0 * cells);
-#define CC(M, F) k_coarse_cycle<M, F><<<1, CC_T, 0, c.stream>>>(a)
+#define CC(M, F) k_coarse_cycle<M, F><<<1, CC_T, CC_SMEM, c.stream>>>(a)
         if (model == MGG_MODEL_FR) {
             if (frn == 0) CC(MGG_MODEL_FR, 0); else if (frn == 1) CC(MGG_MODEL_FR, 1); else CC(MGG_MODEL_FR, 2);
         } else if (model == MGG_MODEL_DGP) CC(MGG_MODEL_DGP, 0);
@@ -2692,13 +2955,13 @@ void mg_read_report(Ctx& c, mgg_mg_report* rep) {
 }
 
 void mg_alloc(Ctx& c) {
-    // the fused smoother's five-plane ring exceeds the 48 KB default
+    // the fused smoother's ring exceeds the 48 KB default
 #define MGG_FB_ATTR(M, F, L0) \
-    MGG_CUDA(cudaFuncSetAttribute(k_smooth_fused<M, F, L0>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM))
+    MGG_CUDA(cudaFuncSetAttribute(k_smooth_fused<M, F, L0>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb_smem(L0)))
     MGG_FB_ATTR(MGG_MODEL_FR, 0, true); MGG_FB_ATTR(MGG_MODEL_FR, 0, false);
     MGG_FB_ATTR(MGG_MODEL_FR, 1, true); MGG_FB_ATTR(MGG_MODEL_FR, 1, false);
 #define MGG_FB_ATTRX(M, F, L0) \
-    MGG_CUDA(cudaFuncSetAttribute(k_smooth_fused<M, F, L0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM))
+    MGG_CUDA(cudaFuncSetAttribute(k_smooth_fused<M, F, L0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb_smem(L0)))
     MGG_FB_ATTRX(MGG_MODEL_FR, 0, true); MGG_FB_ATTRX(MGG_MODEL_FR, 0, false);
     MGG_FB_ATTRX(MGG_MODEL_FR, 1, true); MGG_FB_ATTRX(MGG_MODEL_FR, 1, false);
     MGG_FB_ATTRX(MGG_MODEL_FR, 2, true); MGG_FB_ATTRX(MGG_MODEL_FR, 2, false);
@@ -2707,6 +2970,12 @@ void mg_alloc(Ctx& c) {
     MGG_FB_ATTR(MGG_MODEL_FR, 2, true); MGG_FB_ATTR(MGG_MODEL_FR, 2, false);
     MGG_FB_ATTR(MGG_MODEL_SYMMETRON, 0, true); MGG_FB_ATTR(MGG_MODEL_SYMMETRON, 0, false);
 #undef MGG_FB_ATTR
+#define MGG_CC_ATTR(M, F) \
+    MGG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<M, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, CC_SMEM))
+    MGG_CC_ATTR(MGG_MODEL_FR, 0); MGG_CC_ATTR(MGG_MODEL_FR, 1); MGG_CC_ATTR(MGG_MODEL_FR, 2);
+    MGG_CC_ATTR(MGG_MODEL_DGP, 0); MGG_CC_ATTR(MGG_MODEL_KMOUFLAGE, 0); MGG_CC_ATTR(MGG_MODEL_CSF, 0);
+    MGG_CC_ATTR(MGG_MODEL_SYMMETRON, 0);
+#undef MGG_CC_ATTR
     const int N = c.N;
     int levelmax = 0;
     while ((1 << levelmax) < N) ++levelmax;
