@@ -18,6 +18,7 @@
 // pass, which is deterministic.
 #include "mgg_internal.cuh"
 #include "reduce.cuh"
+#include <cooperative_groups.h>
 #include <cmath>
 #include <cstdlib>
 #include <map>
@@ -2187,28 +2188,35 @@ int tune_chunk(Ctx& c, int kind, int n, int variant, int dflt, const std::vector
 }
 
 // ---------------------------------------------------- small levels --------
-// The cycle below a level of at most 16^3 cells (MGG_COARSE_N lowers the size;
-// 0 turns it off) in one launch of one block: the host lists the level
-// operations in the order vcycle / fcycle / wcycle issue them (the colour
+// The cycle below a level of at most 32^3 cells (MGG_COARSE_N lowers the size;
+// 0 turns it off) in one launch of one cluster of blocks: the host lists the
+// level operations in the order vcycle / fcycle / wcycle issue them (the colour
 // sweeps of the smoothing, the residual, the restriction, the FAS right-hand
-// side, the correction), and the block makes one pass over the level's cells
-// per operation with the per-cell code of the separate kernels, a block
-// barrier between passes.  All of those levels' arrays (131 KB from 16^3 down)
-// live in shared memory: the passes are a few hundred to two thousand cells,
-// bound by latency, and each used to wait for L2 twice.
-constexpr int CC_T = 1024, CC_MAXOPS = 384, CC_MAXLEV = 4, CC_MAXN = 16;
-constexpr int CC_CELLS = 4096 + 512 + 64 + 8, CC_SMEM = 7 * CC_CELLS * (int)sizeof(float);
+// side, the correction), and the cluster makes one pass over the level's cells
+// per operation with the per-cell code of the separate kernels.  Levels of 16^3
+// cells and more run on all of the cluster's threads, their arrays in global
+// memory (L2), a cluster barrier between passes; the smaller ones on its first
+// block, their arrays in shared memory, a block barrier between passes.  As
+// separate launches these levels cost tens of launch latencies per cycle and left
+// the GPU idle; on one block the passes over 16^3 cells (and more so 32^3) were
+// bound by one SM's instruction rate (ncu: 0.57 of its issue slots).  Against one
+// block up to 16^3 and separate launches above: a batch of eight 128^3 boxes 13.4 ->
+// 11.5 ms for three steps, a W-cycle solve at 256^3 14.7 -> 14.3 ms, eight steps at
+// 64^3 unchanged at 4.3 ms (a V-cycle from 32^3 down 78 us here).  8 blocks of 512
+// threads: 4.75 ms for the latter; 8 of 1024 spill; 16 of 256: 4.53 ms.
+constexpr int CL_N = 16, CL_T = 512;
+constexpr int CC_MAXOPS = 384, CC_MAXLEV = 5, CC_MAXN = 32, CC_BLOCKN = 8;
+constexpr int CC_CELLS = 512 + 64 + 8;   // of the levels in shared memory
 enum : uint8_t { CO_RED = 0, CO_BLACK = 1, CO_RESID, CO_RESTRICT, CO_RHS, CO_PROLONG };
-struct CoarseArgs {
-    int nops, n;                             // n: cells per edge of level 0 (of the list)
-    uint8_t op[CC_MAXOPS], lev[CC_MAXOPS];   // lev: level index relative to the first
-    float* u;                                // the first level's field (in and out), density and right-hand side
-    const float *d, *tau;
-    LevelConsts K[CC_MAXLEV];
-};
 struct CoarseLev {
     int n;
     float *u, *d, *tau, *res, *rr, *ru, *snap;
+};
+struct CoarseArgs {
+    int nops, ncl;                           // ncl: levels that run on the whole cluster
+    uint8_t op[CC_MAXOPS], lev[CC_MAXOPS];   // lev: level index relative to the first
+    CoarseLev g[CC_MAXLEV];                  // the levels' arrays in global memory
+    LevelConsts K[CC_MAXLEV];
 };
 // level l (of n >> l cells per edge) in shared memory
 __device__ __forceinline__ CoarseLev coarse_level(float* sm, int n, int l) {
@@ -2239,42 +2247,59 @@ __device__ __forceinline__ void coarse_relax(const CoarseLev& L, const LevelCons
     }
 }
 
+// one operation of level L (C: the next coarser level; k, kn: their constants)
 template <int MODEL, int FRN>
-__global__ void __launch_bounds__(CC_T) k_coarse_cycle(const __grid_constant__ CoarseArgs a) {
-    extern __shared__ __align__(16) float sm[];
-    const uint32_t t = threadIdx.x, st = CC_T;
-    const int n3 = a.n * a.n * a.n;
-    {
-        const CoarseLev L = coarse_level(sm, a.n, 0);
-        for (int e = t; e < n3; e += st) {
-            L.u[e] = a.u[e];
-            L.d[e] = a.d[e];
-            L.tau[e] = a.tau[e];
-        }
-    }
-    __syncthreads();
-    for (int o = 0; o < a.nops; ++o) {
-        const int l = a.lev[o], op = a.op[o];
-        const CoarseLev L = coarse_level(sm, a.n, l);
-        if (op <= CO_BLACK) {
-            coarse_relax<MODEL, FRN>(L, a.K[l], op, t, st);
-        } else if (op == CO_RESID) {
-            resid_cells<MODEL, FRN, false>(L.u, L.d, L.tau, L.res, L.n, a.K[l], t, st);
-        } else if (op == CO_RESTRICT) {   // level l -> l + 1
-            const CoarseLev C = coarse_level(sm, a.n, l + 1);
-            restrict_cells(L.res, L.u, L.d, C.n, C.rr, C.ru, C.u, C.d, t, st);
-        } else if (op == CO_RHS) {
-            rhs_cells<MODEL, FRN>(L.ru, L.d, L.rr, L.tau, L.n, a.K[l], t, st);
-        } else {   // CO_PROLONG: correct level l from level l + 1
-            const CoarseLev C = coarse_level(sm, a.n, l + 1);
-            prolong_cells(L.u, C.u, C.ru, L.n, MODEL, a.K[l + 1].phibar, a.K[l + 1].ctl2, t, st);
-        }
-        __syncthreads();
-    }
-    for (int e = t; e < n3; e += st) a.u[e] = sm[e];   // the first level's field starts the shared memory
+__device__ __forceinline__ void coarse_op(int op, const CoarseLev& L, const CoarseLev& C, const LevelConsts& k,
+                                          const LevelConsts& kn, uint32_t t, uint32_t st) {
+    if (op <= CO_BLACK) coarse_relax<MODEL, FRN>(L, k, op, t, st);
+    else if (op == CO_RESID) resid_cells<MODEL, FRN, false>(L.u, L.d, L.tau, L.res, L.n, k, t, st);
+    else if (op == CO_RESTRICT) restrict_cells(L.res, L.u, L.d, C.n, C.rr, C.ru, C.u, C.d, t, st);
+    else if (op == CO_RHS) rhs_cells<MODEL, FRN>(L.ru, L.d, L.rr, L.tau, L.n, k, t, st);
+    else prolong_cells(L.u, C.u, C.ru, L.n, MODEL, kn.phibar, kn.ctl2, t, st);
 }
 
-// size limit of the one-block cycle (cells per edge)
+template <int MODEL, int FRN>
+__global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T) k_coarse_cycle(const __grid_constant__ CoarseArgs a) {
+    __shared__ __align__(16) float sm[7 * CC_CELLS];
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const uint32_t t = threadIdx.x, gt = blockIdx.x * CL_T + t;
+    const CoarseLev& B = a.g[a.ncl];   // the first level in shared memory
+    const int b3 = B.n * B.n * B.n;
+    bool below = false;   // the first block has worked on the levels below since the last cluster barrier
+    for (int o = 0; o < a.nops; ++o) {
+        const int l = a.lev[o], op = a.op[o];
+        if (l < a.ncl) {
+            if (below) {   // the correction comes next: the field of the first level below back to global memory
+                if (blockIdx.x == 0)
+                    for (int e = t; e < b3; e += CL_T) B.u[e] = sm[e];
+                cl.sync();
+                below = false;
+            }
+            coarse_op<MODEL, FRN>(op, a.g[l], a.g[l + 1], a.K[l], a.K[l + 1], gt, CL_N * CL_T);
+            cl.sync();
+        } else {
+            if (blockIdx.x == 0) {
+                const CoarseLev L = coarse_level(sm, B.n, l - a.ncl);
+                if (!below) {   // after the restriction: the first level below into shared memory
+                    for (int e = t; e < b3; e += CL_T) {
+                        L.u[e] = B.u[e];
+                        L.d[e] = B.d[e];
+                        L.rr[e] = B.rr[e];
+                        L.ru[e] = B.ru[e];
+                    }
+                    __syncthreads();
+                }
+                coarse_op<MODEL, FRN>(op, L, coarse_level(sm, B.n, l - a.ncl + 1), a.K[l], a.K[l + 1], t, CL_T);
+                __syncthreads();
+            }
+            below = true;
+        }
+    }
+    if (below && blockIdx.x == 0)   // a list that starts below (NGRID = 16)
+        for (int e = t; e < b3; e += CL_T) B.u[e] = sm[e];
+}
+
+// size limit of the one-launch cycle (cells per edge)
 int coarse_max_n() {
     static const int v = [] {
         const char* e = std::getenv("MGG_COARSE_N");
@@ -2465,9 +2490,9 @@ struct Solver {
         return grid_for((int64_t)n * n * n);
     }
 
-    // level-0 residual norm: the per-block partials and their fixed-order sum into
-    // out (device), without waiting; the RMS residual is sqrt(*out / n^3)
-    void norm0_async(double* out) {
+    // level-0 residual norm: the per-block partials in c.red_partial; returns their
+    // number.  The RMS residual is the root of their sum (in order) over n^3.
+    int norm0_partials() {
         const LevelConsts k = make_consts(c, 0);
         const int n = k.n;
         const int64_t work = (int64_t)n * n * n;
@@ -2482,7 +2507,7 @@ struct Solver {
                 launch_resid<true>(0, k, nb);
             }
         }
-        reduce_sum_blocks_async(c, nb, out);
+        return nb;
     }
 
     double resid(int l) {
@@ -2491,7 +2516,7 @@ struct Solver {
         const int64_t work = (int64_t)n * n * n;
         const int g = grid_for(work);
         if (l == 0) {
-            norm0_async(c.red_out);
+            reduce_sum_blocks_async(c, norm0_partials(), c.red_out);
             MGG_CUDA(cudaMemcpyAsync(c.h_red, c.red_out, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
             MGG_CUDA(cudaStreamSynchronize(c.stream));
             return sqrt(c.h_red[0] / pow((double)n, 3));
@@ -2560,6 +2585,7 @@ struct Solver {
             k_restrict<<<g, 256, 0, c.stream>>>(F.res, F.u, F.d, n, L.rr, L.ru, L.u, L.d);
             MGG_CHECK_LAUNCH();
         }
+        if (coarse_first(lc)) return;   // its right-hand side is the first operation of the one-launch cycle
         if (march_ok(n)) {
             auto launch = [&](int z) {
                 march<OPM_RHS>(kc, L.ru, L.d, L.rr, L.tau, dim3(n / OP_X, n / OP_Y, n / z), z);
@@ -2643,27 +2669,28 @@ struct Solver {
         o.add(CO_PROLONG, l);
         emit_smooth(o, l);
     }
+    bool coarse_first(int l) const {   // level l starts the one-launch cycle
+        const int lim = coarse_max_n(), n = c.N >> l;
+        return l >= 1 && lim > 0 && n <= lim && (l == 1 || (c.N >> (l - 1)) > lim);
+    }
     bool coarse_cycle(int l, int type) {
-        const int lim = coarse_max_n();
-        const int n = c.N >> l;
-        if (l < 1 || lim <= 0 || n > lim || (l > 1 && (c.N >> (l - 1)) <= lim) || n >= OP_X) return false;
+        if (!coarse_first(l)) return false;
         CoarseArgs a;
         memset(&a, 0, sizeof(a));
         OpList o{a, l};
+        o.add(CO_RHS, l);
         emit_cycle(o, l, type);
-        if (!o.ok) return false;
+        if (!o.ok) throw Error{MGG_ERR_STATE, "scalar_field: the one-launch cycle does not fit its list"};
         double cells = 0.0;
-        a.n = n;
-        a.u = c.lev[l].u;
-        a.d = c.lev[l].d;
-        a.tau = c.lev[l].tau;
         for (int q = l; q <= c.levelmax && q - l < CC_MAXLEV; ++q) {
             const Level& V = c.lev[q];
+            a.g[q - l] = CoarseLev{V.n, V.u, V.d, V.tau, V.res, V.rr, V.ru, V.snap};
             a.K[q - l] = make_consts(c, q);
+            if (V.n > CC_BLOCKN) a.ncl = q - l + 1;
             cells += (double)V.n * V.n * V.n;
         }
         ProfScope ps(c, K_MG_COARSE, 16.0 * 4.0 * cells);
-#define CC(M, F) k_coarse_cycle<M, F><<<1, CC_T, CC_SMEM, c.stream>>>(a)
+#define CC(M, F) k_coarse_cycle<M, F><<<CL_N, CL_T, 0, c.stream>>>(a)
         if (model == MGG_MODEL_FR) {
             if (frn == 0) CC(MGG_MODEL_FR, 0); else if (frn == 1) CC(MGG_MODEL_FR, 1); else CC(MGG_MODEL_FR, 2);
         } else if (model == MGG_MODEL_DGP) CC(MGG_MODEL_DGP, 0);
@@ -2758,15 +2785,20 @@ __global__ void k_mg_loop_reset(MgLoopState* st) {
 }
 
 // The exit test of scalar_field (PMP2extradof.f90:107-121) after one cycle, on the
-// device, from the fixed-order sum of the level-0 squared residuals.  The double
+// device, from the level-0 squared residuals' partial sums, added in a fixed order.  The double
 // arithmetic is the host loop's (division and square root are correctly rounded
 // on both sides), so the residuals, the cycle count and the exit reason are the
 // host loop's bit for bit.  Sets the condition of the enclosing while node:
 // 1 runs another cycle, 0 ends the solve.  A non-finite residual ends it too
 // (and, with sticky non-null, sets bit 3 of *sticky).
-__global__ void k_mg_exit(const double* __restrict__ sum, double n3, MgLoopState* st, int iter_max,
-                          double res_conv, int32_t* sticky, cudaGraphConditionalHandle h) {
-    const double res = sqrt(sum[0] / n3);
+__global__ void __launch_bounds__(1024) k_mg_exit(const double* __restrict__ part, int npart, double n3,
+                                                  MgLoopState* st, int iter_max, double res_conv, int32_t* sticky,
+                                                  cudaGraphConditionalHandle h) {
+    double sum = 0.0;   // as reduce_sum_blocks_async
+    for (int i = threadIdx.x; i < npart; i += blockDim.x) sum += part[i];
+    sum = block_sum_fixed(sum);
+    if (threadIdx.x != 0) return;
+    const double res = sqrt(sum / n3);
     const int iter = st->iter + 1;
     st->iter = iter;
     bool can_exit = false;
@@ -2934,8 +2966,8 @@ bool mg_record_solve(Ctx& c, int i_step, Recorder& rec, MgLoopState* slot, int32
     MGG_CHECK_LAUNCH();
     rec.loop([&](cudaGraphConditionalHandle h) {
         run_cycle(g, s);
-        s.norm0_async(c.red_out);
-        k_mg_exit<<<1, 1, 0, c.stream>>>(c.red_out, n3, slot, g.iter_count_max, g.res_conv, sticky, h);
+        const int np = s.norm0_partials();
+        k_mg_exit<<<1, 1024, 0, c.stream>>>(c.red_partial, np, n3, slot, g.iter_count_max, g.res_conv, sticky, h);
         MGG_CHECK_LAUNCH();
     });
     mg_exit_rescale(c);
@@ -2970,8 +3002,8 @@ void mg_alloc(Ctx& c) {
     MGG_FB_ATTR(MGG_MODEL_FR, 2, true); MGG_FB_ATTR(MGG_MODEL_FR, 2, false);
     MGG_FB_ATTR(MGG_MODEL_SYMMETRON, 0, true); MGG_FB_ATTR(MGG_MODEL_SYMMETRON, 0, false);
 #undef MGG_FB_ATTR
-#define MGG_CC_ATTR(M, F) \
-    MGG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<M, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, CC_SMEM))
+    // clusters of more than eight blocks are opted into
+#define MGG_CC_ATTR(M, F) MGG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<M, F>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
     MGG_CC_ATTR(MGG_MODEL_FR, 0); MGG_CC_ATTR(MGG_MODEL_FR, 1); MGG_CC_ATTR(MGG_MODEL_FR, 2);
     MGG_CC_ATTR(MGG_MODEL_DGP, 0); MGG_CC_ATTR(MGG_MODEL_KMOUFLAGE, 0); MGG_CC_ATTR(MGG_MODEL_CSF, 0);
     MGG_CC_ATTR(MGG_MODEL_SYMMETRON, 0);
@@ -3039,8 +3071,8 @@ void mg_scalar_field(Ctx& c, int i_step, mgg_mg_report* rep, bool defer) {
         const double n3 = pow((double)c.N, 3);
         auto capture_body = [&](cudaGraphConditionalHandle h) {
             run_cycle();
-            s.norm0_async(c.red_out);
-            k_mg_exit<<<1, 1, 0, c.stream>>>(c.red_out, n3, c.mg_loop, g.iter_count_max, g.res_conv, nullptr, h);
+            const int np = s.norm0_partials();
+            k_mg_exit<<<1, 1024, 0, c.stream>>>(c.red_partial, np, n3, c.mg_loop, g.iter_count_max, g.res_conv, nullptr, h);
             MGG_CHECK_LAUNCH();
         };
         // capture into body (an existing graph) or, with body null, into a new graph
