@@ -23,6 +23,7 @@
 #include "mgg_internal.cuh"
 #include "fft.cuh"
 #include <map>
+#include <mutex>
 #include "reduce.cuh"
 
 namespace mgg {
@@ -364,35 +365,25 @@ __global__ void __launch_bounds__(XShape<N, C>::NT, fft_min_blocks<typename XSha
 // C: the arithmetic type of the lines (float2, or double2 for the plain path's
 // FP64 line arithmetic); the spectrum is stored as float2 either way.
 
-// the warp's sum of v, modulo 2^64, from its 22-bit pieces (27 bits each when summed)
-__device__ __forceinline__ unsigned long long warp_sum64(unsigned long long v) {
-    const uint32_t s0 = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0x3fffffu);
-    const uint32_t s1 = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 22) & 0x3fffffu);
-    const uint32_t s2 = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 44));
-    return (unsigned long long)s0 + ((unsigned long long)s1 << 22) + ((unsigned long long)s2 << 44);
+// LM_POWER's fixed-point sums of a block, per pair of (linear, log) bin: a value of
+// up to 2^61 is added as three 32-bit words (19, 19 and the remaining bits: a block
+// has at most 8192 modes, so the lower words cannot overflow, and the upper word's
+// sum is right modulo 2^26, all of it that the 64-bit sum keeps), each one
+// shared-memory operation that nothing waits for.  The 64-bit adds it replaces are
+// compare-and-swap loops, which had to be summed over a warp first, a handful of
+// distinct bins one after the other: z pass of P(k) at 512^3 (plain path, a late
+// snapshot) 2.70 -> 0.93 ms.
+__device__ __forceinline__ void limb_add(uint32_t* h, int npair, int p, unsigned long long v) {
+    atomicAdd(h + p, (uint32_t)v & 0x7ffffu);
+    atomicAdd(h + npair + p, (uint32_t)(v >> 19) & 0x7ffffu);
+    atomicAdd(h + 2 * npair + p, (uint32_t)(v >> 38));
 }
-// Adds v to h0[b0] and h1[b1], and q to h2[b0] when quad, for every lane of the warp
-// (all 32 lanes call it together): the 32 modes a warp bins at once mostly fall in a
-// few shells, so the lanes of each distinct (b0, b1) are summed by warp reductions
-// and one lane adds the sums with one shared-memory atomic each.  The histograms are
-// integers (fixed point), so the totals do not depend on the order of the additions.
-__device__ __forceinline__ void warp_bin_add(unsigned long long* h0, unsigned long long* h1, unsigned long long* h2,
-                                             int b0, int b1, unsigned long long v, unsigned long long q, bool quad) {
-    const int lane = threadIdx.x & 31, key = b0 << 8 | b1;   // b1 < 256 (the log-bin table's bytes)
-    unsigned rem = __ballot_sync(0xffffffffu, v != 0ull || q != 0ull);
-    while (rem) {
-        const int lead = __ffs(rem) - 1;
-        const bool mine = key == __shfl_sync(0xffffffffu, key, lead);
-        const unsigned long long t = warp_sum64(mine ? v : 0ull);
-        const unsigned long long tq = quad ? warp_sum64(mine ? q : 0ull) : 0ull;
-        if (lane == lead) {
-            atomicAdd(h0 + b0, t);
-            atomicAdd(h1 + b1, t);
-            if (quad) atomicAdd(h2 + b0, tq);
-        }
-        rem &= ~__ballot_sync(0xffffffffu, mine);
-    }
+__device__ __forceinline__ unsigned long long limb_sum(const uint32_t* h, int npair, int p) {
+    return (unsigned long long)h[p] + ((unsigned long long)h[npair + p] << 19) + ((unsigned long long)h[2 * npair + p] << 38);
 }
+
+// entries of the bin table before its pairs (an even number, so that the pairs are aligned)
+__host__ __device__ constexpr int bin_table_m2(int N) { return (3 * (N / 2) * (N / 2) + 2) / 2 * 2; }
 
 template <int N, class C>
 struct LShape {   // y / z lines: TX kx columns x N elements per block
@@ -464,48 +455,54 @@ __global__ void __launch_bounds__(LShape<N, C>::NT, fft_min_blocks<typename LSha
 #pragma unroll
         for (int i = 0; i < F::E; ++i) put(i, elem_of<F, F::FIRST>(t, i));
     } else {   // LM_POWER
-        // linear bins, log bins, quadrupole-weighted linear bins (two's-complement sums).
-        // Whole warps bin together: one shared-memory atomic per distinct bin of a warp.
-        unsigned long long* hl = reinterpret_cast<unsigned long long*>(sm_raw + S::WORDS * sizeof(C));
-        unsigned long long* hg = hl + (N + 1);
-        unsigned long long* hq = hl + 2 * (N + 1);
-        const int nh = ex.quad ? 3 * (N + 1) : 2 * (N + 1);
-        for (int e = threadIdx.x; e < nh; e += NT) hl[e] = 0ull;
+        // linear bins, log bins, quadrupole-weighted linear bins (two's-complement sums)
+        static_assert(TX * N <= 8192, "limb_add");
+        uint32_t* hl = reinterpret_cast<uint32_t*>(sm_raw + S::WORDS * sizeof(C));
+        uint32_t* hq = hl + 3 * ex.npair;
+        const int nh = (ex.quad ? 6 : 3) * ex.npair;
+        for (int e = threadIdx.x; e < nh; e += NT) hl[e] = 0u;
         __syncthreads();
         fft_regs<-1, F, false, 1, TX, S::PADU, true, false>(v, s, t, tw);
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < F::E; ++i) s[elem_of<F, F::LAST>(t, i) * TX] = v[i];   // read back by this thread only
         const int ky = o;
+        const double w = ((kx == 0 || kx == N / 2) ? 1.0 : 2.0) * ex.amp_scale;   // amp_scale times a power of two
 #pragma unroll 1
         for (int i = 0; i < F::E; ++i) {
             const int kz = elem_of<F, F::LAST>(t, i);
             const C f = s[kz * TX];
             const int my = ky <= N / 2 ? ky : N - ky, mz = kz <= N / 2 ? kz : N - kz;
             const int m2 = kx * kx + my * my + mz * mz;
-            int MP = 0, ML = 0;
-            unsigned long long fx = 0ull, fq = 0ull;
-            if (valid && m2 != 0) {
+            if (!valid || m2 == 0) continue;
+            const int p = __ldg(ex.bins + m2);
+            const double amp = ((double)f.x * f.x + (double)f.y * f.y) * w;
+            const unsigned long long fx = __double2ull_rn(amp);
+            if (fx == 0ull) continue;   // and so is its quadrupole, smaller by |P2| <= 1
+            limb_add(hl, ex.npair, p, fx);
+            if (ex.quad) {
+                // P2(mu) about z in Real*4 as the reference (cosmu2 = MI/RK**2, P2 = 1.5 cosmu2 - 0.5,
+                // PMP2mod_power.f90:386-388, its MI being the z index after its x<->z transposition)
                 const float RK = sqrtf((float)m2);
-                MP = (int)(RK + 0.5f);
-                MP = MP < 1 ? 1 : MP;
-                ML = __ldg(ex.logbin + m2);
-                const double w = (kx == 0 || kx == N / 2) ? 1.0 : 2.0;
-                const double amp = w * ((double)f.x * f.x + (double)f.y * f.y) * ex.amp_scale;
-                fx = __double2ull_rn(amp);
-                if (ex.quad) {
-                    // P2(mu) about z in Real*4 as the reference (cosmu2 = MI/RK**2, P2 = 1.5 cosmu2 - 0.5,
-                    // PMP2mod_power.f90:386-388, its MI being the z index after its x<->z transposition)
-                    const float cosmu2 = __fdiv_rn((float)(mz * mz), __fmul_rn(RK, RK));
-                    const float p2 = __fsub_rn(__fmul_rn(1.5f, cosmu2), 0.5f);
-                    fq = (unsigned long long)__double2ll_rn(amp * (double)p2);
-                }
+                const float cosmu2 = __fdiv_rn((float)(mz * mz), __fmul_rn(RK, RK));
+                const float p2 = __fsub_rn(__fmul_rn(1.5f, cosmu2), 0.5f);
+                limb_add(hq, ex.npair, p, (unsigned long long)__double2ll_rn(amp * (double)p2));
             }
-            warp_bin_add(hl, hg, hq, MP, ML, fx, fq, ex.quad != 0);
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < nh; e += NT)
-            if (hl[e]) atomicAdd(ex.hist + e, hl[e]);
+        const ushort2* pair = reinterpret_cast<const ushort2*>(ex.bins + bin_table_m2(N));
+        for (int p = threadIdx.x; p < ex.npair; p += NT) {
+            const unsigned long long a = limb_sum(hl, ex.npair, p);
+            const ushort2 b = __ldg(pair + p);
+            if (a) {
+                atomicAdd(ex.hist + b.x, a);
+                atomicAdd(ex.hist + (N + 1) + b.y, a);
+            }
+            if (ex.quad) {
+                const unsigned long long q = limb_sum(hq, ex.npair, p);
+                if (q) atomicAdd(ex.hist + 2 * (N + 1) + b.x, q);
+            }
+        }
     }
 }
 
@@ -563,7 +560,7 @@ void lines_c(const FftPlan& p, const C* tw, float2* buf, int axis, int mode, con
     case LM_INV: k_fft_lines<LM_INV, N, C><<<grid, S::NT, smem, s>>>(buf, estride, ostride, tw, ex); break;
     case LM_GREEN: k_fft_lines<LM_GREEN, N, C><<<grid, S::NT, smem, s>>>(buf, estride, ostride, tw, ex); break;
     case LM_POWER:
-        smem += 3 * (size_t)(N + 1) * sizeof(unsigned long long);
+        smem += (ex.quad ? 6 : 3) * (size_t)ex.npair * sizeof(uint32_t);
         k_fft_lines<LM_POWER, N, C><<<grid, S::NT, smem, s>>>(buf, estride, ostride, tw, ex);
         break;
     case LM_DISP:
@@ -648,21 +645,48 @@ double2* make_twiddles64(int N) {
     return d;
 }
 
-// log-bin table per integer |k|^2 with the reference's Real*4 arithmetic
-// (MPlog = max(1, min(NPOWER, INT(Log10(RK)/dLog + 1000.) - 1000)), PMP2mod_power.f90:396)
-uint8_t* make_logbins(int N) {
+// Bins per integer |k|^2 with the reference's Real*4 arithmetic: linear
+// MP = max(INT(RK + 0.5), 1), log MPlog = max(1, min(NPOWER, INT(Log10(RK)/dLog +
+// 1000.) - 1000)) (PMP2mod_power.f90:396), and the distinct pairs of them (few, since
+// both grow with |k|): pair index per |k|^2, then (linear, log) per pair.
+struct BinTable {
+    std::vector<uint16_t> table;
+    int npair = 0;
+    int lin(int m2) const { return table[m2bins + 2 * table[m2]]; }
+    int log(int m2) const { return table[m2bins + 2 * table[m2] + 1]; }
+    int m2bins = 0;
+};
+static BinTable bin_table(int N) {
     const int m2max = 3 * (N / 2) * (N / 2);
-    std::vector<uint8_t> lb(m2max + 1, 0);
+    BinTable b;
+    b.m2bins = bin_table_m2(N);
+    b.table.assign(b.m2bins, 0);
+    std::vector<uint16_t> pairs;
+    int last = -1;
     for (int m2 = 1; m2 <= m2max; ++m2) {
         const float RK = sqrtf((float)m2);
+        int mp = (int)(RK + 0.5f);
+        mp = mp < 1 ? 1 : mp;
         int ml = (int)(log10f(RK) / 0.02f + 1000.0f) - 1000;
         ml = ml < 1 ? 1 : (ml > N ? N : ml);
         if (ml > 255) ml = 255;
-        lb[m2] = (uint8_t)ml;
+        if (last < 0 || pairs[2 * last] != mp || pairs[2 * last + 1] != ml) {
+            pairs.push_back((uint16_t)mp);
+            pairs.push_back((uint16_t)ml);
+            ++last;
+        }
+        b.table[m2] = (uint16_t)last;
     }
-    uint8_t* d = nullptr;
-    MGG_CUDA(cudaMalloc(&d, m2max + 1));
-    MGG_CUDA(cudaMemcpy(d, lb.data(), m2max + 1, cudaMemcpyHostToDevice));
+    b.npair = last + 1;
+    b.table.insert(b.table.end(), pairs.begin(), pairs.end());
+    return b;
+}
+
+uint16_t* make_bins(int N) {
+    const BinTable b = bin_table(N);
+    uint16_t* d = nullptr;
+    MGG_CUDA(cudaMalloc(&d, sizeof(uint16_t) * b.table.size()));
+    MGG_CUDA(cudaMemcpy(d, b.table.data(), sizeof(uint16_t) * b.table.size(), cudaMemcpyHostToDevice));
     return d;
 }
 
@@ -684,7 +708,7 @@ void fft_alloc(Ctx& c) {
     }
     MGG_CUDA(cudaMalloc(&c.green, sizeof(double) * N));
     MGG_CUDA(cudaMemcpy(c.green, g.data(), sizeof(double) * N, cudaMemcpyHostToDevice));
-    c.pk_logbin = make_logbins(N);
+    c.pk_bins = make_bins(N);
     MGG_CUDA(cudaMalloc(&c.pk_hist, sizeof(unsigned long long) * 3 * (N + 1)));
     fft_set_attributes();
 }
@@ -760,7 +784,40 @@ static void mode_counts(int N, std::vector<double>& cnt) {
     }
 }
 
-void power_bins(Ctx& c, const float* grid, int N, const float2* tw, const double2* tw64, const uint8_t* logbin,
+namespace {
+// Mode counts and sums of |k| per linear and log bin: they depend on the mesh size alone
+// (powers of two up to 1024), so they are formed once per size and process (2 ms of
+// host time at 512^3, as much as the transform, when every call did).
+struct BinCounts {
+    std::vector<double> iV, dk, iVl, dkl;
+    int npair = 0;   // of the bin table
+};
+const BinCounts& bin_counts(int N) {
+    static std::mutex mu;
+    static std::map<int, BinCounts> all;
+    std::lock_guard<std::mutex> lk(mu);
+    BinCounts& b = all[N];
+    if (!b.iV.empty()) return b;
+    std::vector<double> cnt;
+    mode_counts(N, cnt);
+    const BinTable bt = bin_table(N);
+    BinCounts r;
+    r.npair = bt.npair;
+    for (auto* v : {&r.iV, &r.dk, &r.iVl, &r.dkl}) v->assign(N + 1, 0.0);
+    for (size_t m2 = 1; m2 < cnt.size(); ++m2) {
+        if (cnt[m2] == 0.0) continue;
+        const float RK = sqrtf((float)m2);
+        const int MP = bt.lin((int)m2), ML = bt.log((int)m2);
+        r.iV[MP] += cnt[m2];
+        r.dk[MP] += cnt[m2] * (double)RK;
+        r.iVl[ML] += cnt[m2];
+        r.dkl[ML] += cnt[m2] * (double)RK;
+    }
+    return b = std::move(r);
+}
+}  // namespace
+
+void power_bins(Ctx& c, const float* grid, int N, const float2* tw, const double2* tw64, const uint16_t* bins,
                 bool quad, PkBins& out) {
     const double cells = (double)N * N * N;
     // Parseval bound for the fixed-point scale: sum_k |delta_k|^2 = sum delta^2 / N^3
@@ -785,7 +842,9 @@ void power_bins(Ctx& c, const float* grid, int N, const float2* tw, const double
     p.tw = tw;
     p.tw64 = tw64;
     LineExtra ex;
-    ex.logbin = logbin;
+    const BinCounts& bc = bin_counts(N);   // exact, data independent
+    ex.bins = bins;
+    ex.npair = bc.npair;
     ex.hist = c.pk_hist;
     ex.amp_scale = scale / (cells * cells);
     ex.quad = quad ? 1 : 0;
@@ -807,23 +866,7 @@ void power_bins(Ctx& c, const float* grid, int N, const float2* tw, const double
     std::vector<unsigned long long> h(nh);
     MGG_CUDA(cudaMemcpyAsync(h.data(), c.pk_hist, sizeof(unsigned long long) * nh, cudaMemcpyDeviceToHost, c.stream));
     MGG_CUDA(cudaStreamSynchronize(c.stream));
-    // mode counts and <k> per bin (exact, data independent)
-    static thread_local std::map<int, std::vector<double>> counts;
-    std::vector<double>& cnt = counts[N];
-    if (cnt.empty()) mode_counts(N, cnt);
-    std::vector<double> iV(N + 1, 0.0), dk(N + 1, 0.0), iVl(N + 1, 0.0), dkl(N + 1, 0.0);
-    std::vector<uint8_t> lb(cnt.size());
-    MGG_CUDA(cudaMemcpy(lb.data(), logbin, cnt.size(), cudaMemcpyDeviceToHost));
-    for (size_t m2 = 1; m2 < cnt.size(); ++m2) {
-        if (cnt[m2] == 0.0) continue;
-        const float RK = sqrtf((float)m2);
-        int MP = (int)(RK + 0.5f);
-        MP = MP < 1 ? 1 : MP;
-        iV[MP] += cnt[m2];
-        dk[MP] += cnt[m2] * (double)RK;
-        iVl[lb[m2]] += cnt[m2];
-        dkl[lb[m2]] += cnt[m2] * (double)RK;
-    }
+    const std::vector<double>&iV = bc.iV, &dk = bc.dk, &iVl = bc.iVl, &dkl = bc.dkl;
     const float Pi = 3.141592653f;
     const float Scale = 2.0f * Pi / c.cfg.box;
     const float b3 = c.cfg.box * c.cfg.box * c.cfg.box;
@@ -850,7 +893,7 @@ void power_spectrum(Ctx& c, int nbins, double* k_out, double* n_out, double* p_o
                     double* nl_out, double* pl_out) {
     BucketScope bs(c, MGG_T_POWER);
     PkBins b;
-    power_bins(c, c.fi, c.N, c.tw_n, c.cfg.precision == MGG_PREC_PLAIN ? c.tw64_n : nullptr, c.pk_logbin, false, b);
+    power_bins(c, c.fi, c.N, c.tw_n, c.cfg.precision == MGG_PREC_PLAIN ? c.tw64_n : nullptr, c.pk_bins, false, b);
     for (int I = 1; I <= nbins && I <= c.N / 2; ++I) {
         if (k_out) k_out[I - 1] = b.k[I];
         if (n_out) n_out[I - 1] = b.n[I];

@@ -30,7 +30,8 @@ struct LineExtra {
     const double* green = nullptr;   // G(k) per complex index, length n
     double green_scale = 0.0;        // trfi * 2 / n^3
     // LM_POWER
-    const uint8_t* logbin = nullptr;        // log bin per integer |k|^2
+    const uint16_t* bins = nullptr;         // bin table of make_bins: pair per integer |k|^2, then the pairs
+    int npair = 0;
     unsigned long long* hist = nullptr;     // [3][n+1] fixed-point sums (linear, log, quadrupole)
     double amp_scale = 0.0;                 // fixed-point scale * 1/n^6
     int quad = 0;                           // also the P2(mu)-weighted linear sums (hist[2][..])
