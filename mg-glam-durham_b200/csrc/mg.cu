@@ -1712,7 +1712,7 @@ __device__ __forceinline__ void restrict1_cell(const UA& U, const DA& Dn, const 
         double Q;
         if (MODEL == MGG_MODEL_DGP) {   // PMP2MGsolver_DGP.f90:467-716, Eq. (B1) form
             Q = -8.0 * kc.dg_fct2;
-#pragma unroll 1
+#pragma unroll
             for (int m = 0; m < 8; ++m) {
                 const int a = m & 1, b = (m >> 1) & 1, c = m >> 2;
                 const float X = U(a + 1, b, c) + U(a - 1, b, c);
@@ -1730,7 +1730,7 @@ __device__ __forceinline__ void restrict1_cell(const UA& U, const DA& Dn, const 
             }
         } else if (MODEL == MGG_MODEL_KMOUFLAGE) {   // PMP2MGsolver_kmf.f90:507-1067
             Q = 0.0;
-#pragma unroll 1
+#pragma unroll
             for (int m = 0; m < 8; ++m) {
                 const int a = m & 1, b = (m >> 1) & 1, c = m >> 2;
                 Nb19 v;
@@ -1745,7 +1745,7 @@ __device__ __forceinline__ void restrict1_cell(const UA& U, const DA& Dn, const 
             }
         } else if (MODEL == MGG_MODEL_CSF) {   // PMP2MGsolver_csf.f90:355-572
             Q = 0.0;
-#pragma unroll 1
+#pragma unroll
             for (int m = 0; m < 8; ++m) {
                 const int a = m & 1, b = (m >> 1) & 1, c = m >> 2;
                 double phi, A_phi, V_phi;
@@ -1810,6 +1810,9 @@ __global__ void k_restrict1(const float* __restrict__ fi, const float* __restric
 constexpr int RS_CX = 32, RS_CY = 8, RS_FX = 2 * RS_CX + 2, RS_FY = 2 * RS_CY + 2, RS_FPL = RS_FX * RS_FY;
 
 // five blocks (40 warps) per SM; the 19-point k-mouflage needs more registers; the
+// children of the nDGP, k-mouflage and csf restriction are unrolled, which turns their
+// neighbours' shared-memory offsets into constants (all launches of the class at 512^3
+// and below, nDGP 0.231 -> 0.205 ms on average, k-mouflage 0.272 -> 0.251); the
 // precision form's f(R) n = 1 restriction at seven blocks (32 registers): 0.546 ->
 // 0.455 ms per launch at 1024^3 against five (48 registers); six 0.502
 template <int MODEL, int FRN, bool MIX>

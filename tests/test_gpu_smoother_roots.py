@@ -1,6 +1,7 @@
 """The fused smoother's roots where they are hard: a nearly empty box with a few very dense cells, so that the first sweeps
 leave the FP32 Newton region (cells whose value falls by orders of magnitude, negative starts after a correction) and the
-closed form takes over, against the serial FP64-arithmetic oracle.  128^3 is the smallest mesh with the fused sweep.
+closed form takes over, against the serial FP64-arithmetic oracle.  128^3 is the smallest mesh with the fused sweep, 64^3
+the one whose levels take the tile sweep on the finest level.
 
 Bounds: those of the other solves, 1e-5 of the field's maximum on the plain path and 1e-4 in the precision form."""
 import numpy as np
@@ -8,12 +9,11 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-N = 128
 
-
+@pytest.mark.parametrize("N", [64, 128])
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("model,n,cycle", [(1, 0, "V"), (1, 1, "V"), (1, 1, "W"), (1, 2, "V"), (3, 1, "V")])
-def test_dense_cells_in_a_void(orc, model, n, cycle, precision):
+def test_dense_cells_in_a_void(orc, model, n, cycle, precision, N):
     import mgglam_b200 as m
 
     cfg = m.make_config(N, 16, float(N), mg_model=model, fr_n=n, fr0=-1e-6, cycle=cycle, iter_count_max=2,
