@@ -2146,6 +2146,17 @@ int forced_chunk() {
     return forced;
 }
 
+// The candidates of level l: a 128^3 level has 8 tiles of 128 x 16 cells, so chunks of
+// 8 and 4 planes are what it takes to reach the GPU's 148 SMs (four f(R) steps at
+// 256^3, plain path, 16.7 -> 15.6 ms, at 512^3, precision form, 71.3 -> 69.8 ms).  The
+// finest level of a 128^3 box keeps the longer ones: their halo planes are work that
+// boxes run side by side would pay for (eight of them 11.8 -> 12.8 ms with short ones,
+// one alone 0.88 -> 0.75 ms per solve).
+std::vector<int> chunks(std::vector<int> c, int l, int n) {
+    if (l > 0 && n <= 128) c.insert(c.begin(), c.front() > 8 ? std::initializer_list<int>{4, 8} : std::initializer_list<int>{4});
+    return c;
+}
+
 template <class F>
 int tune_chunk(Ctx& c, int kind, int n, int variant, int dflt, const std::vector<int>& cands, F&& launch) {
     const int f = forced_chunk();
@@ -2354,7 +2365,8 @@ struct Solver {
                 MGG_CHECK_LAUNCH();
             };
 #undef SWEEP
-            launch(tune_chunk(c, TK_SWEEP, n, model * 2 + (mix ? 1 : 0), march_cz(n), {8, 16, 32, 64}, launch));
+            launch(tune_chunk(c, TK_SWEEP, n, model * 4 + (l == 0 ? 2 : 0) + (mix ? 1 : 0), march_cz(n),
+                              chunks({8, 16, 32, 64}, l, n), launch));
         } else if (model == MGG_MODEL_DGP || model == MGG_MODEL_KMOUFLAGE) {
             // same-colour diagonal neighbours read the field as it was before this
             // sweep: red U -> snap, black snap -> U (relax is called in red/black pairs)
@@ -2389,7 +2401,7 @@ struct Solver {
         const int n = k.n;
         const bool mix = c.cfg.precision == MGG_PREC_MIXED;
         const int cz = tune_chunk(c, TK_FUSED, n, model * 100 + frn * 10 + (l == 0 ? 2 : 0) + (mix ? 1 : 0),
-                                  n >= 256 ? 64 : (n >= 128 ? 32 : 16), {16, 32, 64, 128},
+                                  n >= 256 ? 64 : (n >= 128 ? 32 : 16), chunks({16, 32, 64, 128}, l, n),
                                   [&](int z) { fused_launch(l, k, uin, uout, z); });
         fused_launch(l, k, uin, uout, cz, true);
     }
@@ -2528,7 +2540,7 @@ struct Solver {
             auto launch = [&](int z) {
                 march<OPM_RES>(k, U(l), D(l), c.lev[l].tau, c.lev[l].res, dim3(n / OP_X, n / OP_Y, n / z), z);
             };
-            const int zt = tune_chunk(c, TK_MARCH, n, march_variant(OPM_RES), march_cz(n), {8, 16, 32, 64}, launch);
+            const int zt = tune_chunk(c, TK_MARCH, n, march_variant(OPM_RES), march_cz(n), chunks({8, 16, 32, 64}, 1, n), launch);
             ProfScope ps(c, K_MG_RESID, 16.0 * (double)work);
             launch(zt);
             return 0.0;
@@ -2593,7 +2605,7 @@ struct Solver {
             auto launch = [&](int z) {
                 march<OPM_RHS>(kc, L.ru, L.d, L.rr, L.tau, dim3(n / OP_X, n / OP_Y, n / z), z);
             };
-            const int zt = tune_chunk(c, TK_MARCH, n, march_variant(OPM_RHS), march_cz(n), {8, 16, 32, 64}, launch);
+            const int zt = tune_chunk(c, TK_MARCH, n, march_variant(OPM_RHS), march_cz(n), chunks({8, 16, 32, 64}, 1, n), launch);
             ProfScope ps(c, K_MG_RHS, 16.0 * (double)work);
             launch(zt);
         } else {
@@ -2621,7 +2633,7 @@ struct Solver {
         const LevelConsts k = make_consts(c, lc);
         ProfScope ps(c, K_MG_PROLONG, 8.0 * (double)work + 1.0 * (double)work);
         if (nf >= PR_X) {
-            const int czf = PR_CZF;
+            const int czf = nf > PR_X || lc == 1 ? PR_CZF : 4;   // a 128^3 level has 16 tiles: short chunks (see chunks)
             const bool mix = c.cfg.precision == MGG_PREC_MIXED;   // FP32 in the precision form
             if (mix)
                 k_prolong_march<true><<<dim3(nf / PR_X, nf / PR_Y, nf / czf), PR_T, 0, c.stream>>>(
