@@ -89,13 +89,14 @@ __global__ void k_cic_scatter(const float* __restrict__ x, const float* __restri
 // lists; two adds that nothing waits for); FIX_CARRY, the low and high 32 bits, the
 // carry taken from the low word's old value; FIX_BIG the same for v >= 2^51 (a
 // handful of particles on the whole mesh).  Below 2^51 the integer is read off the
-// sum v + 2^52, which rounds as the conversion does.
+// sum v + 2^52, which rounds as the conversion does; the sum is a call of its own, or the
+// compiler would fuse it with v's last product, whose rounding is part of the weight.
 enum FixMode { FIX_SPLIT, FIX_CARRY, FIX_BIG };
 constexpr float kBigWpar = 131072.0f;   // particle weight from which v can reach 2^51
 template <FixMode MODE>
 __device__ __forceinline__ void fix_add(uint32_t* lo, uint32_t* hi, int cell, double v) {
     const unsigned long long b = MODE == FIX_BIG ? __double2ull_rn(v)
-                                                 : (unsigned long long)__double_as_longlong(v + 4503599627370496.0);
+                                                 : (unsigned long long)__double_as_longlong(__dadd_rn(v, 4503599627370496.0));
     const uint32_t l = (uint32_t)b, hw = (uint32_t)(b >> 32);
     if (MODE == FIX_SPLIT) {
         atomicAdd(lo + cell, l & 0xfffffu);

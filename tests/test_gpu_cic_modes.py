@@ -56,3 +56,40 @@ def test_deposit_is_the_integer_sum(n, nrow, kind):
     for c, q in expected(*parts[:3], n).items():
         ref[c] = np.float32(q / 2.0 ** 32 - 1.0)
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
+# T3, T1, T2 in units of 2^-23 whose product lies within 2^-22 of a half in units of 2^-32, on the other side of it than
+# the product rounded to FP64: rounded once (a product and a sum contracted into one operation) it is another integer.
+TIES = [(7158006, 6728658, 6458770), (7057203, 6570542, 6373546), (7000868, 7953007, 6098447),
+        (7925127, 7701376, 6431604), (6732247, 5993096, 7800782), (6210210, 7201439, 6547712)]
+
+
+@pytest.mark.parametrize("crowd", ["elsewhere", "same row"])   # short and long lists
+@pytest.mark.parametrize("t", TIES)
+def test_weights_are_rounded_as_products(t, crowd):
+    """One particle with such a weight, another that fills its cell up to 1 within 2^-23 (so that FP32 holds the sum's last
+    bit), the rest on nodes."""
+    import mgglam_b200 as m
+
+    n = 32
+    t3, t1, t2 = (a / 2.0 ** 23 for a in t)
+    far = 1.0 if crowd == "same row" else 10.0
+    x, y, z = (np.full(n ** 3, v, np.float32) for v in (10.0, far, far))
+    x[0], y[0], z[0] = 2 - t1, 2 - t2, 2 - t3
+    x[1], y[1], z[1] = 1 + np.rint(t3 * t1 * t2 * 2 ** 23) / 2 ** 23, 1, 1
+    assert x[0] == 2 - t1 and y[0] == 2 - t2 and z[0] == 2 - t3
+    product = t3 * t1 * (t2 * 2.0 ** 32)
+    assert int(np.rint(product)) != (t[0] * t[1] * t[2] + 2 ** 36) // 2 ** 37
+    box = m.Box(m.make_config(n, n, float(n), mg_flag=0))
+    try:
+        box.upload_particles(x, y, z, *[np.zeros_like(x)] * 3)
+        box.set_time(0.5, 0.01)
+        box.density()
+        got = box.download_grid(m.GRID_FI)
+    finally:
+        box.close()
+    ref = np.full(n ** 3, -1.0, np.float32)
+    for c, q in expected(x, y, z, n).items():
+        ref[c] = np.float32(q / 2.0 ** 32 - 1.0)
+    assert abs(ref[0]) < 2 ** -23
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
