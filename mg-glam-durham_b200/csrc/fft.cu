@@ -198,7 +198,7 @@ __device__ __forceinline__ void dft(C* v) {
 // measured copy bandwidth), plain path at 512^3: x 0.965 -> 0.311 ms (0.53) and
 // 1.014 -> 0.299, y 0.799 -> 0.305 (0.54), z with the Green's multiply 1.391 ->
 // 0.555 (0.30); precision form at 1024^3: x 3.76 -> 1.62 ms (0.81) and 4.01 ->
-// 1.77, y 2.11 -> 1.90 (0.69), z 4.81 -> 3.56 (0.37; two transforms of a pencil at
+// 1.77, y 2.11 -> 1.90 (0.69), z 4.81 -> 3.50 (0.38; two transforms of a pencil at
 // 16 warps per SM).  Staging the next pencil by tensor copies, as the y and z
 // passes did, is worth less than the registers' shorter path.
 //
@@ -444,12 +444,7 @@ __global__ void __launch_bounds__(LShape<N, C>::NT, fft_min_blocks<typename LSha
         for (int i = 0; i < F::E; ++i) {
             double A1 = (go + gx) + __ldg(ex.green + elem_of<F, F::LAST>(t, i));
             if (fabs(A1) < 1.0e-7) A1 = 1.0;
-            // green_scale / A1: SFU reciprocal seed (2^-22) refined by Newton steps in FP64, two for
-            // FP64 lines, one (2^-44) for FP32 lines (|A1| lies in [1e-7, 12], a normal float)
-            double r = (double)__fdividef(1.0f, (float)A1);
-            r = fma(r, fma(-A1, r, 1.0), r);
-            if (sizeof(C) == 16) r = fma(r, fma(-A1, r, 1.0), r);
-            v[i] = cscale(v[i], (T)(ex.green_scale * r));
+            v[i] = cscale(v[i], (T)(ex.green_scale * green_reciprocal(A1)));
         }
         fft_regs<1, F, true, 1, TX, S::PADU, true, true>(v, s, t, tw);
 #pragma unroll

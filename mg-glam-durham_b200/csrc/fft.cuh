@@ -2,9 +2,25 @@
 // initial-condition generator.
 #pragma once
 #include <cuda_runtime.h>
+#include <cmath>
 #include <cstdint>
 
 namespace mgg {
+
+// 1 / A1 of the Poisson kernel, |A1| in [1e-7, 12]: an FP32 seed and two Newton steps
+// in FP64 (2^-22 -> 2^-44 -> FP64 rounding), for FP32 lines too: the product with
+// green_scale is then rounded once, to the lines' type.  The seed is the short
+// division: the exact one branches, and the butterflies around it wait (z pass at
+// 512^3 in FP32 lines 0.360 -> 0.485 ms).
+__host__ __device__ __forceinline__ double green_reciprocal(double A1) {
+#ifdef __CUDA_ARCH__
+    double r = (double)__fdividef(1.0f, (float)A1);
+#else
+    double r = (double)(1.0f / (float)A1);
+#endif
+    r = fma(r, fma(-A1, r, 1.0), r);
+    return fma(r, fma(-A1, r, 1.0), r);
+}
 
 // A 3-D real <-> half-complex transform of an n^3 grid.
 //   real grid : n^3 floats, x fastest
