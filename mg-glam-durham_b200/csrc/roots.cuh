@@ -169,14 +169,18 @@ __host__ __device__ __forceinline__ float quartic_root_newton32(float u, float P
     return nan32();
 }
 
-// FP64 root of the plain path from an FP32 seed: two chord steps, each of which
-// multiplies the relative error by ~1e-6 (see chord_refine); NaN when the seed is
-// unusable or sits near a double root.
+// FP64 root of the plain path from an FP32 seed u0 by two chord steps.  The seed's error
+// e0 is FP32 rounding of terms up to 9 u^3 over the slope f' (cubic; the quartic with one
+// more power of u), so below 1e-6 where f' > u^2; a chord step multiplies an error by
+// about 6 e0 u^2 / f', so two leave FP64 rounding.  Returns NaN where the slope is smaller
+// (towards a double root, where two steps do not do: that takes Q > 0, which the
+// symmetron's coarse levels can have) or negative (not the largest root), and where
+// FP32 underflow may have spoilt the seed (u^3 or u^4 below 1e-30).
 template <bool QUARTIC>
 __host__ __device__ __forceinline__ double refine_seed(float u0, double P, double Q) {
     const float u2 = u0 * u0;
     const float fp = QUARTIC ? fmaf(4.0f * u2, u0, (float)P) : fmaf(3.0f, u2, (float)P);
-    if (!(u0 > 1.0e-15f && fabsf(fp) > 3.0e-3f * (QUARTIC ? u2 * u0 : u2))) return (double)nan32();
+    if (!(u0 > (QUARTIC ? 3.0e-8f : 1.0e-10f) && fp > (QUARTIC ? u2 * u0 : u2))) return (double)nan32();
     const double r = (double)rcp_approx(fp);
     double u = (double)u0;
 #pragma unroll
@@ -211,8 +215,8 @@ __host__ __device__ __attribute__((noinline)) double quartic_root_cold(double P,
 }
 
 // The plain path's cubic (quartic) root from the cell's current value: the FP32
-// Newton root refined in FP64, else the closed form.  The value is the closed form's
-// to FP64 rounding, as before, at a third of its instructions.
+// Newton root refined in FP64, else (NaN) the closed form.  The value is the closed
+// form's to FP64 rounding at a third of its instructions.
 template <bool QUARTIC>
 __host__ __device__ __forceinline__ double root_from(float uold, double P, double Q) {
     const float seed = QUARTIC ? quartic_root_newton32(uold, (float)P, (float)Q)
