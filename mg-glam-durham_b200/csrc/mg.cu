@@ -2126,6 +2126,34 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T) k_coarse_cy
         for (int e = t; e < b3; e += CL_T) B.u[e] = sm[e];
 }
 
+// Clusters of more than eight blocks are opted into, per kernel and device
+template <int MODEL, int FRN>
+bool coarse_opt_in() {
+    return cudaFuncSetAttribute(k_coarse_cycle<MODEL, FRN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+}
+
+// Whether the device runs the cycle's cluster: it takes CL_N free SMs side by side, which
+// a slice of a GPU or an SM limit may not have (asked for one model: a block of any of
+// them fits an SM).  Separate launches serve there.
+bool coarse_fits() {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {CL_N, 1, 1};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CL_N);
+    cfg.blockDim = dim3(CL_T);
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (coarse_opt_in<MGG_MODEL_FR, 0>() && coarse_opt_in<MGG_MODEL_FR, 1>() && coarse_opt_in<MGG_MODEL_FR, 2>() &&
+        coarse_opt_in<MGG_MODEL_DGP, 0>() && coarse_opt_in<MGG_MODEL_KMOUFLAGE, 0>() &&
+        coarse_opt_in<MGG_MODEL_CSF, 0>() && coarse_opt_in<MGG_MODEL_SYMMETRON, 0>() &&
+        cudaOccupancyMaxActiveClusters(&n, k_coarse_cycle<MGG_MODEL_FR, 1>, &cfg) == cudaSuccess)
+        return n > 0;
+    cudaGetLastError();
+    return false;
+}
+
 // size limit of the one-launch cycle (cells per edge)
 int coarse_max_n() {
     static const int v = [] {
@@ -2498,7 +2526,7 @@ struct Solver {
         emit_smooth(o, l);
     }
     bool coarse_first(int l) const {   // level l starts the one-launch cycle
-        const int lim = coarse_max_n(), n = c.N >> l;
+        const int lim = c.coarse_n, n = c.N >> l;
         return l >= 1 && lim > 0 && n <= lim && (l == 1 || (c.N >> (l - 1)) > lim);
     }
     bool coarse_cycle(int l, int type) {
@@ -2830,12 +2858,7 @@ void mg_alloc(Ctx& c) {
     MGG_FB_ATTR(MGG_MODEL_FR, 2, true); MGG_FB_ATTR(MGG_MODEL_FR, 2, false);
     MGG_FB_ATTR(MGG_MODEL_SYMMETRON, 0, true); MGG_FB_ATTR(MGG_MODEL_SYMMETRON, 0, false);
 #undef MGG_FB_ATTR
-    // clusters of more than eight blocks are opted into
-#define MGG_CC_ATTR(M, F) MGG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<M, F>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
-    MGG_CC_ATTR(MGG_MODEL_FR, 0); MGG_CC_ATTR(MGG_MODEL_FR, 1); MGG_CC_ATTR(MGG_MODEL_FR, 2);
-    MGG_CC_ATTR(MGG_MODEL_DGP, 0); MGG_CC_ATTR(MGG_MODEL_KMOUFLAGE, 0); MGG_CC_ATTR(MGG_MODEL_CSF, 0);
-    MGG_CC_ATTR(MGG_MODEL_SYMMETRON, 0);
-#undef MGG_CC_ATTR
+    c.coarse_n = coarse_fits() ? coarse_max_n() : 0;
     const int N = c.N;
     int levelmax = 0;
     while ((1 << levelmax) < N) ++levelmax;

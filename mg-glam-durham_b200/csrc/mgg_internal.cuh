@@ -135,6 +135,7 @@ struct Ctx {
 
     // multigrid arena
     int levelmax = 0, levelmin = 0;
+    int coarse_n = 0;   // levels of at most this many cells per edge run as one launch (0: none)
     Level lev[12];
 
     // FFT workspace: complex half spectrum, padded row pitch nxp (float2 units)

@@ -241,3 +241,46 @@ def test_small_level_cycle_equals_separate_launches(tmp_path):
         for key in out["off"].files:
             a, b = out[tag][key], out["off"][key]
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), (tag, key)
+
+
+_FAKE = """
+extern "C" int cudaOccupancyMaxActiveClusters(int* n, const void*, const void*) {
+    *n = 0;
+    return 0;
+}
+"""
+
+_CLUSTER_SCRIPT = r"""
+import sys, hashlib
+sys.path[:0] = [sys.argv[1], sys.argv[2]]
+import mgglam_b200 as m
+from conftest import random_particles
+b = m.Box(m.make_config(64, 32, 64.0, iter_count_max=2, cycle="W"))
+b.upload_particles(*random_particles(32, 64, seed=2))
+b.set_time(0.7, 0.01)
+b.density()
+b.profile(True)
+b.scalar_field(1)
+print(b.profile_read()["mg_coarse"]["launches"], hashlib.md5(b.download_grid(m.GRID_FI2).tobytes()).hexdigest())
+b.close()
+"""
+
+
+def test_small_levels_without_clusters(tmp_path):
+    """Where no cluster of the small levels' launch fits on the device (its occupancy query answers 0, here a fake of
+    that call), those levels run as separate launches with the same result."""
+    import os
+    import subprocess
+    import sys
+    from conftest import PKG
+    (tmp_path / "fake.cpp").write_text(_FAKE)
+    fake = str(tmp_path / "fake.so")
+    subprocess.run(["g++", "-shared", "-fPIC", "-o", fake, str(tmp_path / "fake.cpp")], check=True)
+    out = []
+    for env in ({}, {"LD_PRELOAD": fake}):
+        r = subprocess.run([sys.executable, "-c", _CLUSTER_SCRIPT, PKG, os.path.dirname(os.path.abspath(__file__))],
+                           env=dict(os.environ, **env), capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-2000:]
+        out.append(r.stdout.split()[-2:])
+    assert int(out[0][0]) > 0 and int(out[1][0]) == 0
+    assert out[0][1] == out[1][1]
