@@ -2035,6 +2035,9 @@ constexpr int CL_N = 16, CL_T = 512;
 constexpr int CC_MAXOPS = 384, CC_MAXLEV = 5, CC_MAXN = 32, CC_BLOCKN = 8;
 constexpr int CC_CELLS = 512 + 64 + 8;   // of the levels in shared memory
 enum : uint8_t { CO_RED = 0, CO_BLACK = 1, CO_RESID, CO_RESTRICT, CO_RHS, CO_PROLONG };
+// operations of a W cycle (the longest) from n^3 cells down, as emit_cycle lists them
+constexpr int coarse_ops(int n) { return n <= 2 ? 4 : 4 + 2 * (3 + coarse_ops(n / 2) + 1 + 4); }
+static_assert(1 + coarse_ops(CC_MAXN) <= CC_MAXOPS && CC_MAXN >> (CC_MAXLEV - 1) == 2, "the list holds any cycle");
 struct CoarseLev {
     int n;
     float *u, *d, *tau, *res, *rr, *ru, *snap;
@@ -2095,6 +2098,7 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T) k_coarse_cy
     bool below = false;   // the first block has worked on the levels below since the last cluster barrier
     for (int o = 0; o < a.nops; ++o) {
         const int l = a.lev[o], op = a.op[o];
+        const int lc = op == CO_RESTRICT || op == CO_PROLONG ? l + 1 : l;   // the last level has none below it
         if (l < a.ncl) {
             if (below) {   // the correction comes next: the field of the first level below back to global memory
                 if (blockIdx.x == 0)
@@ -2102,7 +2106,7 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T) k_coarse_cy
                 cl.sync();
                 below = false;
             }
-            coarse_op<MODEL, FRN>(op, a.g[l], a.g[l + 1], a.K[l], a.K[l + 1], gt, CL_N * CL_T);
+            coarse_op<MODEL, FRN>(op, a.g[l], a.g[lc], a.K[l], a.K[lc], gt, CL_N * CL_T);
             cl.sync();
         } else {
             if (blockIdx.x == 0) {
@@ -2116,7 +2120,7 @@ __global__ void __cluster_dims__(CL_N, 1, 1) __launch_bounds__(CL_T) k_coarse_cy
                     }
                     __syncthreads();
                 }
-                coarse_op<MODEL, FRN>(op, L, coarse_level(sm, B.n, l - a.ncl + 1), a.K[l], a.K[l + 1], t, CL_T);
+                coarse_op<MODEL, FRN>(op, L, coarse_level(sm, B.n, lc - a.ncl), a.K[l], a.K[lc], t, CL_T);
                 __syncthreads();
             }
             below = true;
@@ -2493,9 +2497,7 @@ struct Solver {
     struct OpList {
         CoarseArgs& a;
         int base;
-        bool ok = true;
         void add(uint8_t op, int l) {
-            if (a.nops >= CC_MAXOPS || l - base >= CC_MAXLEV) { ok = false; return; }
             a.op[a.nops] = op;
             a.lev[a.nops] = (uint8_t)(l - base);
             ++a.nops;
@@ -2536,7 +2538,6 @@ struct Solver {
         OpList o{a, l};
         o.add(CO_RHS, l);
         emit_cycle(o, l, type);
-        if (!o.ok) throw Error{MGG_ERR_STATE, "scalar_field: the one-launch cycle does not fit its list"};
         double cells = 0.0;
         for (int q = l; q <= c.levelmax && q - l < CC_MAXLEV; ++q) {
             const Level& V = c.lev[q];
