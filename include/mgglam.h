@@ -303,16 +303,15 @@ int mgg_step(mgg_ctx* ctx, mgg_step_state* st);
  * next while the device runs the last): every step's kernels, each multigrid
  * solve a while node with its exit test on the device, and each step's results
  * (error flags, solve report, kinetic-energy sum) in device memory, read back
- * once after the last step.  No host round trip between the steps.  reports[nsteps] and ekin[nsteps] receive each step's report and
- * ENKIN (either may be NULL); *st is advanced as by nsteps calls of mgg_step,
- * with the same results bit for bit.  A context's first steps, up to and
- * including its first multigrid solve, run one by one (that solve and the
- * first transforms tune the launch shapes), and so do all steps with profiling
- * on, iter_count_max above 1024 or a runtime without conditional graph
- * nodes.  If a step fails,
- * the later steps leave the particles alone, *st is the state after the last
- * good step, and the call returns that step's error; the scalar field is then
- * not meaningful. */
+ * once after the last step.  No host round trip between the steps.
+ * reports[nsteps] and ekin[nsteps] receive each step's report and ENKIN (either
+ * may be NULL); *st is advanced as by nsteps calls of mgg_step, with the same
+ * results bit for bit.  A context's first steps, up to and including its first
+ * multigrid solve, run one by one (that solve tunes the launch shapes), and so
+ * do all steps with profiling on, iter_count_max above 1024 or a runtime
+ * without conditional graph nodes.  If a step fails, the later steps leave the
+ * particles alone, *st is the state after the last good step, and the call
+ * returns that step's error; the scalar field is then not meaningful. */
 int mgg_run_steps(mgg_ctx* ctx, mgg_step_state* st, int32_t nsteps, mgg_mg_report* reports, double* ekin);
 
 /* mgg_step with the particles in host memory: uploads them, runs the step and

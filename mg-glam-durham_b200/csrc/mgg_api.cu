@@ -452,7 +452,6 @@ void step_device(Ctx& c, mgg_step_state* st) {
     st->astep = astep;
     st->istep += 1;
     st->aexpn = st->aexpn + st->astep;   // ADDTIME (256-261)
-    c.stepped = true;
 }
 
 __global__ void k_copy_flags(const int32_t* __restrict__ flags, int32_t* __restrict__ out) { *out = *flags; }
@@ -592,10 +591,9 @@ int mgg_run_steps(mgg_ctx* ctx, mgg_step_state* st, int32_t nsteps, mgg_mg_repor
             while (done < nsteps) one();
             return;
         }
-        // steps run one by one until the context has stepped and solved once: the
-        // first solve (eager) tunes the plane chunks, the first transforms the pencil
-        // width (a symmetron run before a* has no solve until it passes a*)
-        while (done < nsteps && (!c.stepped || (mg && !c.mg_tuned))) one();
+        // steps run one by one until the context has solved once: the first solve (eager)
+        // tunes the plane chunks (a symmetron run before a* has no solve until it passes a*)
+        while (done < nsteps && mg && !c.mg_tuned) one();
         if (done < nsteps)
             run_steps_graphed(c, st, nsteps - done, reports ? reports + done : nullptr, ekin ? ekin + done : nullptr);
     });

@@ -189,7 +189,6 @@ struct Ctx {
     // mgg_run_steps: while a run's graph is recorded, the bucket timers stay off;
     // one result slot per step of the run (device) and their pinned host copy
     bool recording = false;
-    bool stepped = false;   // a main-loop step has run (its transforms tuned the pencil width)
     StepReadback* run_slots = nullptr;
     StepReadback* h_run_slots = nullptr;
     int run_cap = 0;

@@ -160,6 +160,36 @@ def test_run_steps_equals_step_by_step(m, case):
         b.close()
 
 
+_NEWTON_SCRIPT = r"""
+import sys, hashlib
+sys.path.insert(0, sys.argv[1])
+import mgglam_b200 as m
+for queued in (True, False):
+    b = m.Box(m.make_config(64, 32, 64.0, mg_flag=0))
+    b.make_ics(seed=5, aexpn=0.05, astep=0.002)
+    st = b.new_state(0.05, 0.002)
+    if queued:
+        b.run_steps(st, 3)
+    else:
+        for _ in range(3):
+            b.step(st)
+    print(st.istep, st.ekin.hex(), hashlib.md5(b"".join(a.tobytes() for a in b.download_particles())).hexdigest())
+    b.close()
+"""
+
+
+def test_first_steps_of_a_newtonian_run_are_queued():
+    """A run without the scalar field has no solve that tunes: it is recorded from its first step on, also as the first
+    thing a process does, with the result of single steps."""
+    import subprocess
+    import sys
+    from conftest import PKG
+    r = subprocess.run([sys.executable, "-c", _NEWTON_SCRIPT, PKG], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    queued, single = r.stdout.strip().splitlines()[-2:]
+    assert queued == single
+
+
 def test_failed_run_leaves_particles_and_state(m):
     cfg = m.make_config(64, 32, 64.0, mg_model=1, fr_n=1, iter_count_max=3)
     astep0 = m.astep_for_nsteps(A0, 40)
