@@ -221,16 +221,25 @@ import sys
 import numpy as np
 sys.path.insert(0, sys.argv[2])
 import mgglam_b200 as m
-out = {}
+out, tabs = {}, {}
 cases = [("fr1_V", dict(mg_model=1, fr_n=1), 0.05), ("fr0_W", dict(mg_model=1, fr_n=0, cycle="W"), 0.05),
          ("fr2_F", dict(mg_model=1, fr_n=2, cycle="F"), 0.05), ("dgp_V", dict(mg_model=2), 0.05),
          ("sym_W", dict(mg_model=3, cycle="W"), 0.6), ("kmf_F", dict(mg_model=4, cycle="F"), 0.05),
          ("csf_V", dict(mg_model=5), 0.05)]
-for name, kw, a0 in cases:
-    cfg = m.make_config(128, 32, 128.0, iter_count_max=4, **kw)
+runs = [(name, kw, a0, 128, 32) for name, kw, a0 in cases]
+# boxes whose finest level is small: the cycle starts at 16^3 or at 8^3 cells (in one block's shared memory)
+for n in (16, 32):
+    for cycle in "VFW":
+        runs += [("fr%d_%s" % (n, cycle), dict(mg_model=1, fr_n=1, cycle=cycle), 0.05, n, 16),
+                 ("kmf%d_%s" % (n, cycle), dict(mg_model=4, cycle=cycle), 0.05, n, 16)]
+for name, kw, a0, ngrid, nrow in runs:
+    cfg = m.make_config(ngrid, nrow, float(ngrid), iter_count_max=4, **kw)
     tab = None
     if cfg.mg_model in (4, 5):
-        tab, _ = m.background_table(cfg)
+        if cfg.mg_model not in tabs:
+            tabs[cfg.mg_model] = m.background_table(cfg)
+        tab, lam = tabs[cfg.mg_model]
+        cfg.kmf_lambda = cfg.csf_lambda = lam
     b = m.Box(cfg)
     if tab is not None:
         b.set_background(tab)
@@ -250,10 +259,10 @@ np.savez(sys.argv[1], **out)
 
 
 def test_small_level_cycle_equals_separate_launches(tmp_path):
-    """The cycle below 16^3 cells runs as one single-block launch (MGG_COARSE_N=0:
-    as separate launches per level operation; 32: from 32^3 down).  Same per-cell
-    code in the same order of passes: particles, scalar field, residuals and cycle
-    counts after three steps are bit-identical for every model and cycle type."""
+    """The cycle from 32^3 cells down runs as one launch of one cluster (MGG_COARSE_N lowers the size; 0: separate
+    launches per level operation).  Same per-cell code in the same order of passes: particles, scalar field, residuals
+    and cycle counts after three steps are bit-identical for every model and cycle type, wherever the launch starts: on
+    two cluster levels, on one, or in shared memory (8^3 and 4^3)."""
     import os
     import subprocess
     import sys
@@ -261,16 +270,16 @@ def test_small_level_cycle_equals_separate_launches(tmp_path):
     script = tmp_path / "coarse.py"
     script.write_text(_COARSE_SCRIPT)
     out = {}
-    for tag, env in (("off", {"MGG_COARSE_N": "0"}), ("16", {}), ("32", {"MGG_COARSE_N": "32"})):
-        f = tmp_path / f"{tag}.npz"
-        r = subprocess.run([sys.executable, str(script), str(f), PKG], env=dict(os.environ, **env),
+    for limit in (0, 4, 8, 16, 32):
+        f = tmp_path / f"{limit}.npz"
+        r = subprocess.run([sys.executable, str(script), str(f), PKG], env=dict(os.environ, MGG_COARSE_N=str(limit)),
                            capture_output=True, text=True, timeout=900)
         assert r.returncode == 0, r.stderr[-2000:]
-        out[tag] = np.load(f)
-    for tag in ("16", "32"):
-        for key in out["off"].files:
-            a, b = out[tag][key], out["off"][key]
-            assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), (tag, key)
+        out[limit] = np.load(f)
+    for limit in (4, 8, 16, 32):
+        for key in out[0].files:
+            a, b = out[limit][key], out[0][key]
+            assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), (limit, key)
 
 
 _FAKE = """
