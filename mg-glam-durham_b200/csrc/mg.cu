@@ -2478,7 +2478,8 @@ struct Solver {
         const LevelConsts k = make_consts(c, lc);
         ProfScope ps(c, K_MG_PROLONG, 8.0 * (double)work + 1.0 * (double)work);
         if (nf >= PR_X) {
-            const int czf = nf > PR_X || lc == 1 ? PR_CZF : 4;   // a 128^3 level has 16 tiles: short chunks (see chunks)
+            int czf = nf > PR_X || lc == 1 ? PR_CZF : 4;   // a 128^3 level has 16 tiles: short chunks (see chunks)
+            if (forced_chunk() == 4 || forced_chunk() == PR_CZF) czf = forced_chunk();
             const bool mix = c.cfg.precision == MGG_PREC_MIXED;   // FP32 in the precision form
             if (mix)
                 k_prolong_march<true><<<dim3(nf / PR_X, nf / PR_Y, nf / czf), PR_T, 0, c.stream>>>(
