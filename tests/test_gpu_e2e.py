@@ -197,8 +197,8 @@ def test_first_step_1024_headline_configuration(m, orc):
     """Step 1 of the headline configuration (f(R) F5 n = 1, 512^3 particles on a 1024^3
     mesh, L = 1024 Mpc/h, device ICs at a = 0.02, seed 7, the 100-step schedule) on the
     oracle and on the GPU in both forms, routine by routine: the kernels instantiated
-    for 1024^3 (TMA-staged transforms, the marching and fused multigrid kernels on
-    the PM grid) against the reference's arithmetic.  Density within 1e-5, scalar
+    for 1024^3 (the transforms' 1024-point lines, the marching and fused multigrid kernels
+    on the PM grid) against the reference's arithmetic.  Density within 1e-5, scalar
     field and potential within 1e-5 of their maxima (precision form: 1e-4 for the
     field), the same cycle count, positions within 1e-3 cells after MOVE."""
     ngrid, nrow, boxsize, a0 = 1024, 512, 1024.0, 0.02
@@ -319,48 +319,3 @@ def test_potential_512_transform_against_fp64(m, orc, precision):
     print(f"512^3 potential, precision {precision}: against the FP64 transform max {err:.3e} of max|phi|, "
           f"rms {rms:.3e}")
     assert err < (1e-6 if precision == 0 else 1e-5), err
-
-
-_STAGED_SCRIPT = r"""
-import sys, numpy as np
-sys.path[:0] = [sys.argv[2]]
-import mgglam_b200 as m
-n = 256
-rng = np.random.default_rng(13)
-delta = rng.standard_normal(n ** 3, dtype=np.float32)
-delta -= np.float32(delta.mean(dtype=np.float64))
-box = m.Box(m.make_config(n, 16, float(n), mg_flag=0, precision=m.PREC_MIXED))
-box.set_time(0.5, 0.01)
-box.upload_grid(m.GRID_FI, delta)
-box.potential()
-phi = box.download_grid(m.GRID_FI)
-box.upload_grid(m.GRID_FI, delta)
-pk = box.power(recompute_density=False)
-box.close()
-np.savez(sys.argv[1], phi=phi, pk=pk["pk"], pklog=pk["pklog"])
-"""
-
-
-def test_staged_pencils_equal_direct_loads(tmp_path):
-    """The precision form's y / z passes at NGRID >= 256 stage their pencils with
-    tensor copies, 8 or 4 kx columns wide (the autotuner's choice; MGG_FFT_TX
-    forces one); with MGG_FFT_DIRECT=1 they load them directly.  Same
-    arithmetic: the potential and P(k) are bit-identical in all four runs."""
-    import os
-    import subprocess
-    import sys
-    from conftest import PKG
-    script = tmp_path / "staged.py"
-    script.write_text(_STAGED_SCRIPT)
-    out = {}
-    for tag, env in (("tma", {}), ("tx4", {"MGG_FFT_TX": "4"}), ("tx8", {"MGG_FFT_TX": "8"}),
-                     ("direct", {"MGG_FFT_DIRECT": "1"})):
-        f = tmp_path / f"{tag}.npz"
-        r = subprocess.run([sys.executable, str(script), str(f), PKG], env=dict(os.environ, **env),
-                           capture_output=True, text=True, timeout=600)
-        assert r.returncode == 0, r.stderr[-2000:]
-        out[tag] = np.load(f)
-    for tag in ("tma", "tx4", "tx8"):
-        for key in ("phi", "pk", "pklog"):
-            a, b = out[tag][key], out["direct"][key]
-            assert np.array_equal(a, b), (tag, key, float(np.max(np.abs(a.astype(np.float64) - b))))
