@@ -11,10 +11,10 @@
 //   2. scan          : exclusive prefix of the N^2 row counts = row offsets.
 //   3. k_cic_scatter : every particle's position is written to its row bucket
 //                      (a counting sort on the row key).
-//   4. k_cic_deposit : one CTA per 2 x 2 block of output rows.  It walks the source
-//                      rows that can reach its rows in a fixed order, forms the
-//                      reference's FP64 weights, and accumulates them in shared
-//                      memory as 32.32 fixed-point integers.  Integer addition
+//   4. k_cic_deposit : one CTA per 2 x 2 or 4 x 2 block of output rows.  It walks the
+//                      records of the source rows that can reach its rows as one
+//                      list, forms the reference's FP64 weights, and accumulates
+//                      them in shared memory as 32.32 fixed-point integers.  Integer addition
 //                      is associative, so each cell's sum -- and therefore FI --
 //                      is bit-identical for any particle order, launch shape or
 //                      run; the single rounding to FP32 happens at the end.
@@ -87,12 +87,13 @@ __global__ void k_cic_scatter(const float* __restrict__ x, const float* __restri
 // as two 32-bit words: FIX_SPLIT, the low 20 bits and the rest, whose sums cannot
 // overflow while the CTA's list is short and the particles' weight small (most
 // lists; two adds that nothing waits for); FIX_CARRY, the low and high 32 bits, the
-// carry taken from the low word's old value; FIX_BIG the same for v >= 2^51 (a
-// handful of particles on the whole mesh).  Below 2^51 the integer is read off the
-// sum v + 2^52, which rounds as the conversion does; the sum is a call of its own, or the
+// carry taken from the low word's old value; FIX_BIG the same with the integer from
+// the conversion, for particle weights from 2^17 (up to 16 particles on a 128^3 mesh,
+// 8192 on 1024^3).  Below, v is at most 2^49 and the integer is read off the sum
+// v + 2^52, which rounds as the conversion does; the sum is a call of its own, or the
 // compiler would fuse it with v's last product, whose rounding is part of the weight.
 enum FixMode { FIX_SPLIT, FIX_CARRY, FIX_BIG };
-constexpr float kBigWpar = 131072.0f;   // particle weight from which v can reach 2^51
+constexpr float kBigWpar = 131072.0f;   // v <= 2^32 weight, far enough below the 2^52 that the sum needs
 template <FixMode MODE>
 __device__ __forceinline__ void fix_add(uint32_t* lo, uint32_t* hi, int cell, double v) {
     const unsigned long long b = MODE == FIX_BIG ? __double2ull_rn(v)

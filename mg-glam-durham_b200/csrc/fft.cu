@@ -273,7 +273,12 @@ MGG_RAD64(256, 16, 16, 16) MGG_RAD64(512, 16, 16, 16, 2) MGG_RAD64(1024, 16, 16,
 #undef MGG_RAD64
 
 // blocks per SM that the register budget of a line kernel is set for: E complex
-// values, their butterflies and addresses
+// values, their butterflies and addresses.  One rule for every mode; it was set on the
+// plain passes, which do not spill.  The z pass with the Green's multiply holds FP64
+// factors beside its line and spills at some sizes (FP32 lines of 1024 and 256
+// values 0.26 and 0.19 KB, FP64 ones of 256 and 64 0.14 and 0.06 KB, LM_DISP of 512
+// and 1024 24 bytes), at 0.40 to 0.95 of the time of the shared-memory passes
+// it replaced at every size; budgets per mode are not measured.
 template <class F, class C>
 constexpr int fft_min_blocks(int threads) {
     constexpr int words = F::E * (int)sizeof(C) / 4;                    // 32-bit registers of the line

@@ -599,8 +599,8 @@ __global__ void k_relax_sym(float* __restrict__ u, const float* __restrict__ d, 
 // and the two red cells between them are already in registers as their x
 // neighbours, so the four go straight to memory as one 16-byte store.
 //
-// What bounds it is instruction issue (ncu, precision form at 512^3: 0.71 of the
-// slots, 390 warp instructions per warp and plane, 0.37 of DRAM bandwidth); two
+// What bounds it is instruction issue (ncu, precision form at 512^3: 0.69 of the
+// slots, 337 warp instructions per warp and plane, half the copy bandwidth); two
 // blocks of 16 warps at 64 registers, the four cells' roots side by side, do better
 // than three blocks of 21 warps at 32 registers with one root after the other.  Per
 // launch, before -> after: precision form f(R) n = 1 at 1024^3 4.37 -> 4.07 ms (0.48
@@ -2236,7 +2236,7 @@ struct Solver {
         MGG_CHECK_LAUNCH();
     }
 
-    // one red+black iteration in a single fused sweep (7-point models, n >= 64)
+    // one red+black iteration in a single fused sweep (7-point models, n >= 128)
     bool fused_ok(int l) const {
         const int n = c.N >> l;
         return (model == MGG_MODEL_FR || model == MGG_MODEL_SYMMETRON) && n >= FB_X && c.lev[l].snap != nullptr;
